@@ -6,7 +6,7 @@ namespace fe {
 namespace {
 template <int STAGE, int FL, int MP>
 cudaError_t march_list(const MarchMember* mem, const int* bmap, int blocks, cudaStream_t s) {
-  k_march_list<STAGE, 8, FL, MP><<<blocks, dim3(MK, 8), MarchTile<8>::SMEM_BYTES, s>>>(mem, bmap);
+  k_march_list<STAGE, 8, FL, MP><<<blocks, dim3(MT, 8), march_smem_bytes<8, FL>() + sizeof(MarchMember), s>>>(mem, bmap);
   return cudaGetLastError();
 }
 template <int FL>
@@ -46,7 +46,7 @@ cudaError_t batch_set_attrs() {
   auto set = [&](const void* f, int bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   };
-  const int bm = MarchTile<8>::SMEM_BYTES, bs = SgsTile<8>::SMEM_BYTES;
+  const int bm = march_smem_bytes<8, FL_DRY>() + (int)sizeof(MarchMember), bs = SgsTile<8>::SMEM_BYTES;
   set((const void*)k_march_list<0, 8, FL_DRY, -1>, bm);
   set((const void*)k_march_list<1, 8, FL_DRY, -1>, bm);
   set((const void*)k_march_list<2, 8, FL_DRY, -1>, bm);

@@ -17,6 +17,7 @@ inline void phys_from_config(const fe_config& c, Phys& P) {
   P.sj = P.nzh;
   P.si = P.nyh * P.nzh;
   P.n = (long long)P.nxh * P.nyh * P.nzh;
+  P.nc = P.n;
   P.n2 = (long long)P.nxh * P.nyh;
   P.iMin = 3; P.iMax = c.Nx + 3; P.jMin = 3; P.jMax = c.Ny + 3; P.kMin = 3; P.kMax = c.Nz + 3;
   P.dX = c.dX; P.dY = c.dY; P.dZ = c.dZ;
@@ -75,6 +76,13 @@ inline void phys_from_config(const fe_config& c, Phys& P) {
   P.R_gas = c.R_gas; P.R_vapor = c.R_vapor; P.Rv_Rg = c.Rv_Rg; P.cp_gas = c.cp_gas; P.cv_gas = c.cv_gas;
   P.g = c.accel_g; P.R_cp = c.R_cp; P.cp_R = c.cp_R; P.cp_cv = c.cp_cv; P.p0 = c.refPressure; P.kappa = c.kappa;
   P.L_v = c.L_v;
+}
+
+// The padded rows of a domain's own fields (fe_device.cuh).
+inline void phys_pad_rows(Phys& P) {
+  P.sj = (P.nzh + ROW_PAD + 7) / 8 * 8;
+  P.si = P.nyh * P.sj;
+  P.n = (long long)P.nxh * P.si;
 }
 
 }  // namespace fe

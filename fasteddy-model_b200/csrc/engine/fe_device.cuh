@@ -1,8 +1,12 @@
 // fe_device.cuh -- device-side data structures and physics routines of the B200 engine.
 //
-// Layout: every 3-D field is stored exactly as at the C-ABI boundary (reference layout,
-// halo width 3, k fastest): c = i*si + j*sj + k, si = (Ny+6)*(Nz+6), sj = Nz+6. Halo
-// cells are real memory: the periodic images and the vertical boundary values are
+// Layout: a 3-D field has halo width 3 and k fastest, c = i*si + j*sj + k. At the C-ABI boundary
+// (and in the allocation-free call, which works on the caller's arrays) si = (Ny+6)*(Nz+6) and
+// sj = Nz+6. A domain's own fields have padded rows: sj is Nz+6 plus ROW_PAD rounded up to 8
+// floats and a field pointer sits ROW_PAD floats into its row, so that the first interior level of
+// every row starts a 32-byte sector: level pairs move as 8-byte accesses and a (levels x rows) tile
+// as one tensor-map copy, whose rows must start on 16 bytes. The host copies convert (k_pack,
+// k_unpack). Halo cells are real memory: the periodic images and the vertical boundary values are
 // written by the producer of a state (the RK commit epilogue or the halo-fill kernel),
 // so stencils never branch on boundaries. Field f of a state block starts at f*n.
 //
@@ -15,12 +19,15 @@
 
 namespace fe {
 
+constexpr int ROW_PAD = 5;   // floats before level 0 of a padded row (level 3 then starts a sector)
+
 // Scalar configuration of one domain, passed by value to every kernel.
 struct Phys {
   int Nx, Ny, Nz;
   int nxh, nyh, nzh;
   int si, sj;                // i and j strides of a field
-  long long n;               // elements of one halo-inclusive field
+  long long n;               // stride between fields: elements of one field, row padding included
+  long long nc;              // halo-inclusive cells of one field
   long long n2;              // elements of one halo-inclusive 2-D plane
   int iMin, iMax, jMin, jMax, kMin, kMax;
   float dX, dY, dZ, dXi, dYi, dZi;
@@ -76,7 +83,16 @@ struct Ptrs {
   double* lsfPart;             // per-block FP64 partial sums of the slab means
   int *clockIt;                // simTime_it of the step being computed
   float *clockTime;            // simTime of the step being computed
+  int* waitErr;                // set by a kernel whose bounded wait expired (host memory), or nullptr
 };
+
+// Cell t (0..nc-1, row-major over the halo-inclusive extents) as (i, j, k); returns its element index.
+__device__ __forceinline__ long long cell_at(const Phys& P, long long t, int& i, int& j, int& k) {
+  k = (int)(t % P.nzh);
+  j = (int)((t / P.nzh) % P.nyh);
+  i = (int)(t / ((long long)P.nzh * P.nyh));
+  return (long long)i * P.si + (long long)j * P.sj + k;
+}
 
 __device__ __forceinline__ float sgnf(float x) { return copysignf(1.0f, x); }
 
@@ -108,8 +124,13 @@ __device__ __forceinline__ float momentum_bs(const Phys& P, int fld, float z, fl
 }
 
 // ---------------------------------------------------------------- pressure
-// Perturbation pressure of cell t (cuda_pressureDevice.cu:53-113). The moist factor is
-// evaluated with the same double promotions as the reference expression.
+// rho theta (1 + R_v/R_d q_v), q_v in g/kg, formed in double and rounded once as the reference's
+// expression is: an ulp of it is 0.01 Pa of p'.
+__device__ __forceinline__ float moist_rth(float rth, float h) {  // h = R_v/R_d rho q_v / rho
+  return (float)__dmul_rn((double)rth, __fma_rn((double)h, 1e-3, 1.0));
+}
+
+// Perturbation pressure of cell t (cuda_pressureDevice.cu:53-113).
 __device__ __forceinline__ float pert_pressure(const Phys& P, const float* __restrict__ st, const float* __restrict__ pBS,
                                                long long t) {
   const float rt = st[4 * P.n + t];
@@ -117,7 +138,7 @@ __device__ __forceinline__ float pert_pressure(const Phys& P, const float* __res
   if (P.nmoist > 0) {
     const float qv = st[(long long)(5 + P.ntke) * P.n + t];
     const float r = st[t];
-    rtm = (float)((double)rt * (1.0 + (double)(P.Rv_Rg * qv / r) * 1e-3));
+    rtm = moist_rth(rt, __fdiv_rn(__fmul_rn(P.Rv_Rg, qv), r));
   }
   return powf(rtm * P.c1, P.cp_cv) - pBS[t];
 }
@@ -131,7 +152,7 @@ struct Level0 {
 __device__ __forceinline__ Level0 level0_inputs(const Ptrs& Q, long long c0) { return {Q.thBS[c0], Q.rhoBS[c0], Q.pBS[c0]}; }
 __device__ __forceinline__ float level0_pressure(const Phys& P, const Level0& b, int nmoist, float qv) {
   float rt = b.thBS;
-  if (nmoist > 0) rt = (float)((double)rt * (1.0 + (double)(P.Rv_Rg * qv / b.rhoBS) * 1e-3));
+  if (nmoist > 0) rt = moist_rth(rt, __fdiv_rn(__fmul_rn(P.Rv_Rg, qv), b.rhoBS));
   return powf(rt * P.c1, P.cp_cv) - b.pBS;
 }
 __device__ __forceinline__ float level0_pressure(const Phys& P, const Ptrs& Q, long long c0, int nmoist, float qv) {
@@ -167,16 +188,24 @@ struct GlobalPrims {
 // 5th/6th-order hybrid flux across the face between cells s0 (lower) and s1 (upper):
 // arguments are the stencil m2,m1,z0,p1,p2,p3 relative to the lower cell
 // (cuda_advectionDevice.cu:365-376): (37(p1+z0) - 8(p2+m1) + (p3+m2)
-//  - bfac sgn(vel) ((p3-m2) - 5(p2-m1) + 10(p1-z0))) / 60, bfac = 1 - b_hyb >= 0.
+//  - s ((p3-m2) - 5(p2-m1) + 10(p1-z0))) / 60, s = bfac sgn(vel), bfac = 1 - b_hyb >= 0.
+// Evaluated in difference form: with e1 = p1 - z0, e2 = p2 - p1, e3 = p3 - p2, f1 = z0 - m1,
+// f2 = m1 - m2 it is the same polynomial regrouped,
+//   z0 + [(30 - 6s) e1 + (4s - 7) e2 + (1 - s) e3 + (7 + 4s) f1 - (1 + s) f2] / 60,
+// whose five coefficients depend on the face velocity's sign only (the march kernel forms them once per
+// face for all fields) and whose sum adds one rounding at the size of z0 where the sum above has four.
 __device__ __forceinline__ float hyb56_flux(float m2, float m1, float z0, float p1, float p2, float p3, float vel,
                                             float bfac) {
-  const float sixtieth = 1.0f / 60.0f;
-  const float a = __fadd_rn(p1, z0), b = __fadd_rn(p2, m1), c = __fadd_rn(p3, m2);
-  const float d = __fsub_rn(p3, m2), e = __fsub_rn(p2, m1), f = __fsub_rn(p1, z0);
-  const float cen = __fadd_rn(__fmaf_rn(37.0f, a, __fmul_rn(-8.0f, b)), c);
-  const float upw = __fmaf_rn(10.0f, f, __fmaf_rn(-5.0f, e, d));
-  const float sb = copysignf(bfac, vel);  // = bfac sgn(vel) exactly (bfac >= 0)
-  return __fmul_rn(sixtieth, __fmaf_rn(-sb, upw, cen));
+  const float s = copysignf(bfac, vel);  // = bfac sgn(vel) exactly (bfac >= 0)
+  const float c1 = __fmaf_rn(-0.1f, s, 0.5f), c2 = __fmaf_rn(4.0f / 60.0f, s, -7.0f / 60.0f);
+  const float c3 = __fmaf_rn(-1.0f / 60.0f, s, 1.0f / 60.0f), d1 = __fmaf_rn(4.0f / 60.0f, s, 7.0f / 60.0f);
+  const float d2 = __fmaf_rn(-1.0f / 60.0f, s, -1.0f / 60.0f);
+  float t = __fmul_rn(c3, __fsub_rn(p3, p2));
+  t = __fmaf_rn(d2, __fsub_rn(m1, m2), t);
+  t = __fmaf_rn(c2, __fsub_rn(p2, p1), t);
+  t = __fmaf_rn(d1, __fsub_rn(z0, m1), t);
+  t = __fmaf_rn(c1, __fsub_rn(p1, z0), t);
+  return __fadd_rn(z0, t);
 }
 
 // WENO5 face value from the upwind side, stencil a..e (cuda_advectionDevice.cu:626-926).
@@ -297,14 +326,30 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
-__device__ __forceinline__ float2 hyb56_flux2(float2 m2, float2 m1, float2 z0, float2 p1, float2 p2, float2 p3,
-                                              float2 vel, float2 bfac) {
-  const float2 a = add2(p1, z0), b = add2(p2, m1), c = add2(p3, m2);
-  const float2 d = sub2(p3, m2), e = sub2(p2, m1), f = sub2(p1, z0);
-  const float2 cen = add2(fma2(f2s(37.0f), a, mul2(f2s(-8.0f), b)), c);
-  const float2 upw = fma2(f2s(10.0f), f, fma2(f2s(-5.0f), e, d));
-  const float2 msb = f2(-copysignf(bfac.x, vel.x), -copysignf(bfac.y, vel.y));
-  return mul2(f2s(1.0f / 60.0f), fma2(msb, upw, cen));
+// a - b: one packed operation, exact product with -1 (the same rounding as a subtraction)
+__device__ __forceinline__ float2 dif2(float2 a, float2 b) { return __ffma2_rn(b, f2s(-1.0f), a); }
+
+// hyb56_flux() of a lane pair, its coefficients formed apart.
+struct Hyb56 {
+  float2 e1, e2, e3, f1, f2;
+};
+__device__ __forceinline__ Hyb56 hyb56_coef(float2 vel, float bfac) {
+  const float2 s = make_float2(copysignf(bfac, vel.x), copysignf(bfac, vel.y));
+  Hyb56 c;
+  c.e1 = fma2(f2s(-0.1f), s, f2s(0.5f));
+  c.e2 = fma2(f2s(4.0f / 60.0f), s, f2s(-7.0f / 60.0f));
+  c.e3 = fma2(f2s(-1.0f / 60.0f), s, f2s(1.0f / 60.0f));
+  c.f1 = fma2(f2s(4.0f / 60.0f), s, f2s(7.0f / 60.0f));
+  c.f2 = fma2(f2s(-1.0f / 60.0f), s, f2s(-1.0f / 60.0f));
+  return c;
+}
+__device__ __forceinline__ float2 hyb56_face(const Hyb56& c, float2 z0, float2 e1, float2 e2, float2 e3, float2 f1, float2 f2v) {
+  float2 t = mul2(c.e3, e3);
+  t = fma2(c.f2, f2v, t);
+  t = fma2(c.e2, e2, t);
+  t = fma2(c.f1, f1, t);
+  t = fma2(c.e1, e1, t);
+  return add2(z0, t);
 }
 
 template <bool FAST = false>
@@ -339,12 +384,11 @@ __device__ __forceinline__ float2 weno5_flux2(float2 m2, float2 m1, float2 z0, f
                            f2(ux ? p2.x : m1.x, uy ? p2.y : m1.y));
 }
 
-// adv_face() of two stencils (bfac per lane): HYB56 and WENO5 on the packed pipe, the other
-// schemes lane by lane.
+// adv_face() of two stencils (bfac per lane): WENO5 on the packed pipe, the other schemes lane by lane
+// (HYB56 has its own form above).
 template <bool FAST = false>
 __device__ __forceinline__ float2 adv_face2(int sel, float2 m2, float2 m1, float2 z0, float2 p1, float2 p2, float2 p3,
                                             float2 vel, float2 bfac) {
-  if (sel == ADV_HYB56) return hyb56_flux2(m2, m1, z0, p1, p2, p3, vel, bfac);
   if (sel == ADV_WENO5) return weno5_flux2<FAST>(m2, m1, z0, p1, p2, p3, vel);
   return f2(adv_face<FAST>(sel, m2.x, m1.x, z0.x, p1.x, p2.x, p3.x, vel.x, bfac.x),
             adv_face<FAST>(sel, m2.y, m1.y, z0.y, p1.y, p2.y, p3.y, vel.y, bfac.y));
@@ -423,9 +467,6 @@ struct FaceVel {
 __device__ __forceinline__ float contra(float D, float r, float m, float w, float J) {
   return __fmul_rn(__fdiv_rn(D, r), __fmaf_rn(w, J, m));
 }
-// The same with D/rho already formed (one division shared by the three directions).
-__device__ __forceinline__ float contra_dr(float dr, float m, float w, float J) { return __fmul_rn(dr, __fmaf_rn(w, J, m)); }
-__device__ __forceinline__ float contra_z_dr(float dr, float w, float J) { return __fmul_rn(dr, __fmul_rn(w, J)); }
 // Its vertical form (D/rho)*(w*J33).
 __device__ __forceinline__ float contra_z(float D, float r, float w, float J) {
   return __fmul_rn(__fdiv_rn(D, r), __fmul_rn(w, J));

@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -66,6 +67,8 @@ struct fe_domain {
   float* st[3] = {nullptr, nullptr, nullptr};
   float* pr[3] = {nullptr, nullptr, nullptr};
   float* arena = nullptr;                              // the allocation holding st[] and pr[]
+  fe::MarchMaps maps[2][3];                            // stage kernel's tensor maps: tiles of 8 and 4 rows, RK stage
+  int* waitErr = nullptr;                              // mapped host flag: a stage kernel's bounded wait expired
   std::vector<void*> peerMaps;                         // neighbours' arenas opened by IPC handle
   fe_comm* comm = nullptr;                             // stage barrier of a multi-process decomposition
   float* grid = nullptr;
@@ -85,7 +88,9 @@ struct fe_domain {
   int mtj = 8, mni = 64;             // march kernel: rows per tile, planes per thread block
   int sgsNi = 32;                    // fused SGS kernel: planes per thread block
   int sgsRows = 8;                   // fused last-stage physics: rows per tile (8 or 16; 0 = kernel chain)
-  int mniDefault = 64;               // planes per block chosen for the domain size at creation
+  int mniDefault = 64;               // planes per block reported as the default for the domain size
+  int marchSlots = 444;                // thread blocks of 8-row tiles the GPU holds at a time
+  int mniAuto = 0;                   // planes per block launched while the caller has not chosen (0: mni)
   fe_mlp* mlp = nullptr;             // learned SGS closure (nullptr: TKE closure)
   float* feat = nullptr;             // its inputs per ring cell (allocated with the first network)
   cudaGraphExec_t graph = nullptr;
@@ -223,7 +228,10 @@ extern "C" int fe_check_config(const fe_config* c) {
   return FE_OK;
 }
 
-static void make_phys(fe_domain* d) { fe::phys_from_config(d->cfg, d->P); }
+static void make_phys(fe_domain* d) {
+  fe::phys_from_config(d->cfg, d->P);
+  fe::phys_pad_rows(d->P);
+}
 
 static int dev_alloc(fe_domain* d, float** p, size_t nfloats) {
   cudaError_t e = cudaMalloc((void**)p, nfloats * sizeof(float));
@@ -235,6 +243,45 @@ static int dev_alloc(fe_domain* d, float** p, size_t nfloats) {
   CU(cudaMemsetAsync(*p, 0, nfloats * sizeof(float), d->stream));
   return FE_OK;
 }
+
+// Error flags of the domains' kernels, ints in mapped host memory: one page of slots for the process,
+// made on first use (allocating pinned memory for every domain would take milliseconds each), handed
+// out and taken back under a lock.
+namespace {
+class FlagPool {
+ public:
+  int* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!page_ && cudaHostAlloc((void**)&page_, kSlots * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      page_ = nullptr;
+      return nullptr;
+    }
+    for (int s = 0; s < kSlots; s++)
+      if (!used_[s]) {
+        used_[s] = true;
+        page_[s] = 0;
+        return page_ + s;
+      }
+    return nullptr;
+  }
+  void give(int* p) {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (p) used_[p - page_] = false;
+  }
+
+ private:
+  static constexpr int kSlots = 16384;
+  std::mutex mu_;
+  int* page_ = nullptr;
+  bool used_[kSlots] = {};
+};
+FlagPool g_flags;
+}  // namespace
+
+// An allocation of `fields` 3-D fields with padded rows: field f starts at field0(*p) + f * n.
+static int dev_alloc_fields(fe_domain* d, float** p, size_t fields) { return dev_alloc(d, p, (size_t)d->P.n * fields + 8); }
+static float* field0(float* alloc) { return alloc + fe::ROW_PAD; }
 
 static void free_domain(fe_domain* d) {
   if (!d) return;
@@ -250,11 +297,29 @@ static void free_domain(fe_domain* d) {
   cudaFree(d->feat);
   cudaFree(d->clock);
   cudaFree(d->counter);
+  g_flags.give(d->waitErr);
   if (d->fork) cudaEventDestroy(d->fork);
   if (d->join) cudaEventDestroy(d->join);
   if (d->side) cudaStreamDestroy(d->side);
   if (d->stream) cudaStreamDestroy(d->stream);
   delete d;
+}
+
+// Planes per thread block of the march kernel for `cols` tile columns and `slots` resident blocks. A
+// block costs its planes plus about a third of a plane to start; the blocks' planes are latency-bound
+// (a block takes about as long alone as beside others), so small domains want many short blocks and
+// large ones enough waves that the last one is short. Measured stage times against planes per block:
+// 48x40x32 moist 1: 17 us, 2: 26, 8: 80; 128x128x64 dry 2: 95 us, 4: 103, 8: 125, 16: 144;
+// 256x256x128 moist 2: 699 us, 4: 642, 6: 622, 8: 635, 16: 666, 32: 767.
+static int march_planes(long long cols, int nx, long long slots) {
+  int best = 8;
+  double cost = 1e30;
+  for (int ni : {1, 2, 3, 4, 6, 8, 12, 16}) {
+    const double waves = (double)(cols * ((nx + ni - 1) / ni)) / (double)slots;
+    const double c = (std::max(waves, 0.5) + 0.5) * (ni + 1.0 / 3.0);
+    if (c < cost) { cost = c; best = ni; }
+  }
+  return best;
 }
 
 static int march_attrs();
@@ -283,10 +348,8 @@ extern "C" int fe_create(const fe_config* cfg, int device, fe_domain** out) {
   const Phys& P = d->P;
   const size_t n = (size_t)P.n, n2 = (size_t)P.n2;
   {
-    // default march shape: the most planes per thread block of 32 levels x 8 rows (64, 32, 16, 8)
-    // that still leaves 20 waves of two blocks per SM (many blocks balance the SMs, long blocks
-    // amortise each block's first plane: 16 at 512x512x128, 64 at 1024x1024x256, as the
-    // autotuner finds), else 8
+    // reported default march shape: the most planes per thread block of 32 levels x 8 rows (64, 32, 16,
+    // 8) that still leaves 20 waves of two blocks per SM, else 8
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     const long long cols = (long long)((P.Nz + fe::MK - 1) / fe::MK) * ((P.Ny + 7) / 8);
@@ -297,6 +360,8 @@ extern "C" int fe_create(const fe_config* cfg, int device, fe_domain** out) {
         break;
       }
     d->mniDefault = d->mni;
+    d->marchSlots = 3 * nsm;
+    d->mniAuto = march_planes(cols, P.Nx, d->marchSlots);
     // fused SGS kernel (tiles of 32 levels x 8 rows, two blocks per SM): the most planes per block
     // of 64, 32, 16, 8 that still leaves 10 waves
     d->sgsNi = 8;
@@ -313,16 +378,16 @@ extern "C" int fe_create(const fe_config* cfg, int device, fe_domain** out) {
     if (ea == cudaSuccess) ea = fe::batch_set_attrs();
     if (ea != cudaSuccess) rc = set_err(FE_ERR_CUDA, std::string("SGS kernel attributes: ") + cudaGetErrorString(ea));
   }
-  if (rc == FE_OK) rc = dev_alloc(d, &d->arena, 3 * n * (P.nf + 1));
+  if (rc == FE_OK) rc = dev_alloc_fields(d, &d->arena, 3 * (size_t)(P.nf + 1));
   for (int b = 0; b < 3 && rc == FE_OK; b++) {
-    d->st[b] = d->arena + b * n * P.nf;
-    d->pr[b] = d->arena + 3 * n * P.nf + b * n;
+    d->st[b] = field0(d->arena) + b * n * P.nf;
+    d->pr[b] = field0(d->arena) + 3 * n * P.nf + b * n;
   }
   const size_t nsgs = (size_t)(9 + 3 + 1 + 3 * std::max(P.nmoist, 1));
   const size_t nscr = nsgs + (P.turb ? 7 : 0);  // + the march kernel's SGS tendencies
-  if (rc == FE_OK) rc = dev_alloc(d, &d->grid, n * 7);
-  if (rc == FE_OK) rc = dev_alloc(d, &d->base, n * 3);
-  if (rc == FE_OK) rc = dev_alloc(d, &d->scratch, n * nscr);
+  if (rc == FE_OK) rc = dev_alloc_fields(d, &d->grid, 7);
+  if (rc == FE_OK) rc = dev_alloc_fields(d, &d->base, 3);
+  if (rc == FE_OK) rc = dev_alloc_fields(d, &d->scratch, nscr);
   if (rc == FE_OK) rc = dev_alloc(d, &d->surf, n2 * 11);
   const size_t lsfProfBytes = ((size_t)5 * P.nzh * sizeof(float) + 255) / 256 * 256;
   if (rc == FE_OK && P.lsfSub) {
@@ -345,23 +410,42 @@ extern "C" int fe_create(const fe_config* cfg, int device, fe_domain** out) {
     return rc;
   }
   Ptrs& Q = d->Q;
-  Q.zPos = d->grid;
-  Q.J31 = d->grid + n;
-  Q.J32 = d->grid + 2 * n;
-  Q.J33 = d->grid + 3 * n;
-  Q.D = d->grid + 4 * n;
-  Q.invD = d->grid + 5 * n;
-  Q.delta = d->grid + 6 * n;
-  Q.rhoBS = d->base;
-  Q.thBS = d->base + n;
-  Q.pBS = d->base + 2 * n;
-  Q.tau = d->scratch;
-  Q.tkeQ = d->scratch + 9 * n;
-  Q.ls = d->scratch + 12 * n;
-  Q.mtau = d->scratch + 13 * n;
-  Q.sgsF = P.turb ? d->scratch + nsgs * n : nullptr;
+  const float *grid = field0(d->grid), *bs = field0(d->base);
+  float* scr = field0(d->scratch);
+  Q.zPos = grid;
+  Q.J31 = grid + n;
+  Q.J32 = grid + 2 * n;
+  Q.J33 = grid + 3 * n;
+  Q.D = grid + 4 * n;
+  Q.invD = grid + 5 * n;
+  Q.delta = grid + 6 * n;
+  Q.rhoBS = bs;
+  Q.thBS = bs + n;
+  Q.pBS = bs + 2 * n;
+  Q.tau = scr;
+  Q.tkeQ = scr + 9 * n;
+  Q.ls = scr + 12 * n;
+  Q.mtau = scr + 13 * n;
+  Q.sgsF = P.turb ? scr + nsgs * n : nullptr;
   Q.lsfProf = P.lsfSub ? (float*)d->lsfMem : nullptr;
   Q.lsfPart = P.lsfSub ? (double*)((char*)d->lsfMem + lsfProfBytes) : nullptr;
+  for (int t = 0; t < 2 && rc == FE_OK; t++)
+    for (int b = 0; b < 3; b++)
+      if (fe::march_encode_maps(P, Q, t == 0 ? 8 : 4, d->st[b], d->pr[b], d->st[0], &d->maps[t][b]) != cudaSuccess)
+        rc = set_err(FE_ERR_CUDA, "tensor-map encoding failed");
+  void* werr = nullptr;
+  if (rc == FE_OK) {
+    d->waitErr = g_flags.take();
+    if (!d->waitErr || cudaHostGetDevicePointer(&werr, d->waitErr, 0) != cudaSuccess) {
+      cudaGetLastError();
+      rc = set_err(FE_ERR_NOMEM, "no error flag for the domain");
+    }
+  }
+  if (rc != FE_OK) {
+    free_domain(d);
+    return rc;
+  }
+  Q.waitErr = (int*)werr;
   float* s = d->surf;
   Q.cd = s; Q.ch = s + n2; Q.cq = s + 2 * n2; Q.fricVel = s + 3 * n2; Q.htFlux = s + 4 * n2; Q.tskin = s + 5 * n2;
   Q.invOblen = s + 6 * n2; Q.z0m = s + 7 * n2; Q.z0t = s + 8 * n2; Q.qFlux = s + 9 * n2; Q.qskin = s + 10 * n2;
@@ -406,6 +490,51 @@ static int h2d(fe_domain* d, float* dst, const float* src, size_t nfloats) {
   CU(cudaMemcpyAsync(dst, src, nfloats * sizeof(float), cudaMemcpyHostToDevice, d->stream));
   return FE_OK;
 }
+static int d2h(fe_domain* d, float* dst, const float* src, size_t nfloats) {
+  if (!dst) return FE_OK;
+  CU(cudaMemcpyAsync(dst, src, nfloats * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
+  return FE_OK;
+}
+
+// 3-D fields between the host (rows of Nz+6 values) and the domain (padded rows), on the domain's
+// stream: linear copies to or from a staging buffer and one pack or unpack kernel for the fields it
+// holds. The staging buffer is scratch with no content between a step's kernels: the SGS tendencies
+// (written and read within a physics stage) or, without turbulence, the unused TKE flux fields.
+struct FieldCopy {
+  float* dev;   // the field in the domain
+  float* host;
+};
+static int copy_fields(fe_domain* d, const std::vector<FieldCopy>& list, bool toHost) {
+  const Phys& P = d->P;
+  const size_t nc = (size_t)P.nc;
+  float* lin = P.turb ? d->Q.sgsF : d->Q.tkeQ;
+  const size_t cap = std::min<size_t>(P.turb ? 7 : 4, fe::PACK_MAX);
+  const dim3 blk(32, 8);
+  for (size_t at = 0; at < list.size(); at += cap) {
+    const size_t m = std::min(cap, list.size() - at);
+    fe::PackList L;
+    std::memset(&L, 0, sizeof(L));
+    for (size_t q = 0; q < m; q++) L.p[q] = list[at + q].dev;
+    const dim3 g((unsigned)(((long long)P.nxh * P.nyh + 7) / 8), (unsigned)m);
+    if (toHost) fe::k_pack_rows<true><<<g, blk, 0, d->stream>>>(P, L, lin);
+    for (size_t q = 0; q < m;) {
+      size_t run = 1;  // fields that follow one another on the host go in one copy
+      while (q + run < m && list[at + q + run].host == list[at + q].host + run * nc) run++;
+      int rc = toHost ? d2h(d, list[at + q].host, lin + q * nc, run * nc) : h2d(d, lin + q * nc, list[at + q].host, run * nc);
+      if (rc) return rc;
+      q += run;
+    }
+    if (!toHost) fe::k_pack_rows<false><<<g, blk, 0, d->stream>>>(P, L, lin);
+    d->launches++;
+    CU(cudaGetLastError());
+  }
+  return FE_OK;
+}
+static void add_fields(const fe_domain* d, std::vector<FieldCopy>& list, const float* dev, const float* host, size_t nfields) {
+  if (!host) return;
+  for (size_t f = 0; f < nfields; f++)
+    list.push_back({const_cast<float*>(dev) + f * (size_t)d->P.n, const_cast<float*>(host) + f * (size_t)d->P.nc});
+}
 
 static void invalidate_graph(fe_domain* d) {
   if (d->graph) {
@@ -420,14 +549,13 @@ extern "C" int fe_set_grid(fe_domain* d, const float* zPos, const float* J31, co
   if (!d || !zPos || !J31 || !J32 || !J33 || !D_Jac || !invD_Jac) return set_err(FE_ERR_ARG, "NULL argument");
   CU(cudaSetDevice(d->device));
   const size_t n = (size_t)d->P.n;
-  int rc = h2d(d, d->grid, zPos, n);
-  if (!rc) rc = h2d(d, d->grid + n, J31, n);
-  if (!rc) rc = h2d(d, d->grid + 2 * n, J32, n);
-  if (!rc) rc = h2d(d, d->grid + 3 * n, J33, n);
-  if (!rc) rc = h2d(d, d->grid + 4 * n, D_Jac, n);
-  if (!rc) rc = h2d(d, d->grid + 5 * n, invD_Jac, n);
+  float* grid = field0(d->grid);
+  const float* src[6] = {zPos, J31, J32, J33, D_Jac, invD_Jac};
+  std::vector<FieldCopy> list;
+  for (int f = 0; f < 6; f++) add_fields(d, list, grid + f * n, src[f], 1);
+  int rc = copy_fields(d, list, false);
   if (rc) return rc;
-  fe::k_delta<<<(unsigned)((n + 255) / 256), 256, 0, d->stream>>>(d->P, (long long)n, d->grid + 4 * n, d->grid + 6 * n);
+  fe::k_delta<<<(unsigned)((n + 255) / 256), 256, 0, d->stream>>>(d->P, (long long)n, grid + 4 * n, grid + 6 * n);
   d->launches++;
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(d->stream));
@@ -439,11 +567,14 @@ extern "C" int fe_set_base_state(fe_domain* d, const float* bs) {
   if (!d || !bs) return set_err(FE_ERR_ARG, "NULL argument");
   CU(cudaSetDevice(d->device));
   const size_t n = (size_t)d->P.n;
-  int rc = h2d(d, d->base, bs, 2 * n);
+  float* base = field0(d->base);
+  std::vector<FieldCopy> list;
+  add_fields(d, list, base, bs, 2);
+  int rc = copy_fields(d, list, false);
   if (rc) return rc;
   const int thr = 256;
-  fe::k_pbs<<<(unsigned)((n + thr - 1) / thr), thr, 0, d->stream>>>((long long)n, d->base + n, d->P.c1, d->P.cp_cv,
-                                                                    d->base + 2 * n);
+  fe::k_pbs<<<(unsigned)((n + thr - 1) / thr), thr, 0, d->stream>>>((long long)n, base + n, d->P.c1, d->P.cp_cv,
+                                                                    base + 2 * n);
   d->launches++;
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(d->stream));
@@ -495,7 +626,7 @@ extern "C" size_t fe_checkpoint_bytes(const fe_domain* d) {
   if (!d) return 0;
   // with slab-mean subsidence, also the third state buffer: the next forcing step's slab means read
   // its halo cells (the previous step's last-stage input)
-  const size_t ns = (size_t)d->P.nf * (size_t)d->P.n;
+  const size_t ns = (size_t)d->P.nf * (size_t)d->P.nc;
   return sizeof(CkptHeader) + sizeof(float) * (ns + 11 * (size_t)d->P.n2 + (d->P.lsfSub ? ns : 0));
 }
 
@@ -513,10 +644,13 @@ extern "C" int fe_checkpoint_save(fe_domain* d, void* buf, size_t bytes) {
   h.simIt = d->simIt; h.simTime = d->simTime;
   std::memcpy(buf, &h, sizeof(h));
   float* f = reinterpret_cast<float*>(static_cast<char*>(buf) + sizeof(h));
-  const size_t ns = (size_t)d->P.nf * (size_t)d->P.n, n2 = 11 * (size_t)d->P.n2;
-  CU(cudaMemcpyAsync(f, d->st[0], ns * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
-  CU(cudaMemcpyAsync(f + ns, d->surf, n2 * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
-  if (d->P.lsfSub) CU(cudaMemcpyAsync(f + ns + n2, d->st[2], ns * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
+  const size_t ns = (size_t)d->P.nf * (size_t)d->P.nc, n2 = 11 * (size_t)d->P.n2;
+  std::vector<FieldCopy> list;
+  add_fields(d, list, d->st[0], f, d->P.nf);
+  if (d->P.lsfSub) add_fields(d, list, d->st[2], f + ns + n2, d->P.nf);
+  int rc = copy_fields(d, list, true);
+  if (!rc) rc = d2h(d, f + ns, d->surf, n2);
+  if (rc) return rc;
   CU(cudaStreamSynchronize(d->stream));
   return FE_OK;
 }
@@ -536,13 +670,18 @@ extern "C" int fe_checkpoint_load(fe_domain* d, const void* buf, size_t bytes) {
   if (bytes < fe_checkpoint_bytes(d)) return set_err(FE_ERR_ARG, "checkpoint too short");
   CU(cudaSetDevice(d->device));
   const float* f = reinterpret_cast<const float*>(static_cast<const char*>(buf) + sizeof(h));
-  const size_t ns = (size_t)d->P.nf * (size_t)d->P.n, n2 = 11 * (size_t)d->P.n2;
-  CU(cudaMemcpyAsync(d->st[0], f, ns * sizeof(float), cudaMemcpyHostToDevice, d->stream));
-  CU(cudaMemcpyAsync(d->surf, f + ns, n2 * sizeof(float), cudaMemcpyHostToDevice, d->stream));
-  int rc = finish_state(d);
+  const size_t ns = (size_t)d->P.nf * (size_t)d->P.nc, n2 = 11 * (size_t)d->P.n2;
+  std::vector<FieldCopy> list;
+  add_fields(d, list, d->st[0], f, d->P.nf);
+  int rc = copy_fields(d, list, false);
+  if (!rc) rc = h2d(d, d->surf, f + ns, n2);
+  if (!rc) rc = finish_state(d);
   if (rc) return rc;
   if (d->P.lsfSub) {
-    CU(cudaMemcpyAsync(d->st[2], f + ns + n2, ns * sizeof(float), cudaMemcpyHostToDevice, d->stream));
+    list.clear();
+    add_fields(d, list, d->st[2], f + ns + n2, d->P.nf);
+    rc = copy_fields(d, list, false);
+    if (rc) return rc;
     CU(cudaStreamSynchronize(d->stream));
   }
   return fe_set_clock(d, h.simTime, h.simIt);
@@ -580,9 +719,11 @@ extern "C" int fe_set_state(fe_domain* d, const float* hydro, const float* sgstk
   const Phys& P = d->P;
   const size_t n = (size_t)P.n;
   float* A = d->st[0];
-  int rc = h2d(d, A, hydro, 5 * n);
-  if (!rc && P.ntke) rc = h2d(d, A + 5 * n, sgstke, n);
-  if (!rc && P.nmoist) rc = h2d(d, A + (5 + P.ntke) * n, moist, n * P.nmoist);
+  std::vector<FieldCopy> list;
+  add_fields(d, list, A, hydro, 5);
+  if (P.ntke) add_fields(d, list, A + 5 * n, sgstke, 1);
+  if (P.nmoist) add_fields(d, list, A + (5 + P.ntke) * n, moist, P.nmoist);
+  int rc = copy_fields(d, list, false);
   if (rc) return rc;
   return finish_state(d);
 }
@@ -592,9 +733,9 @@ static int finish_state(fe_domain* d) {
   const Phys& P = d->P;
   const size_t n = (size_t)P.n;
   float* A = d->st[0];
-  fe::k_fill<<<blocks1d(P.n, 256), 256, 0, d->stream>>>(P, d->Q, A);
+  fe::k_fill<<<blocks1d(P.nc, 256), 256, 0, d->stream>>>(P, d->Q, A);
   CU(cudaGetLastError());
-  fe::k_pressure<<<blocks1d(P.n, 256), 256, 0, d->stream>>>(P, d->Q, A, d->pr[0]);
+  fe::k_pressure<<<blocks1d(P.nc, 256), 256, 0, d->stream>>>(P, d->Q, A, d->pr[0]);
   CU(cudaGetLastError());
   d->launches += 2;
   // the boundary values that never change (base-state and constant halos) must be valid
@@ -749,7 +890,9 @@ static void launch_stage(const fe_domain* d, cudaStream_t s, const float* cur, c
                          const float* pcur, float* pnxt, float* frhs) {
   const Phys& P = d->P;
   if (d->kind == FE_KERNEL_MARCH) {
-    fe::march_launch<STAGE, MODE>(P, d->Q, d->mtj, d->mni, s, cur, base, nxt, pcur, pnxt, frhs);
+    // a tendency alone is taken of the state A (the maps of stage 0)
+    const fe::MarchMaps& maps = d->maps[d->mtj == 4 ? 1 : 0][MODE == fe::MODE_FRHS ? 0 : STAGE];
+    fe::march_launch<STAGE, MODE>(P, d->Q, maps, d->mtj, d->mniAuto ? d->mniAuto : d->mni, s, cur, base, nxt, pcur, pnxt, frhs);
   } else {
     fe::k_stage<STAGE, MODE><<<stage_grid(d), dim3(d->tk, d->tj, d->ti), 0, s>>>(P, d->Q, cur, base, nxt, pcur, pnxt, frhs);
   }
@@ -835,7 +978,7 @@ extern "C" int fe_advance(fe_domain* d, int nsteps) {
   CU(cudaSetDevice(d->device));
   const bool capture = d->captureFrhs && nsteps > 0;
   if (capture && !d->frhs) {
-    int rc = dev_alloc(d, &d->frhs, (size_t)d->P.n * d->P.nf);
+    int rc = dev_alloc_fields(d, &d->frhs, d->P.nf);
     if (rc) return rc;
   }
   // with tendency capture the last step runs on its own, its last stage storing the tendencies
@@ -852,7 +995,7 @@ extern "C" int fe_advance(fe_domain* d, int nsteps) {
     }
   }
   for (; left > 0; left--) enqueue_step(d, d->stream);
-  if (capture) enqueue_step(d, d->stream, d->frhs);
+  if (capture) enqueue_step(d, d->stream, field0(d->frhs));
   CU(cudaGetLastError());
   for (int s = 0; s < nsteps; s++) {
     d->simTime = d->simTime + d->P.dt;
@@ -861,18 +1004,21 @@ extern "C" int fe_advance(fe_domain* d, int nsteps) {
   return FE_OK;
 }
 
+// Report (and clear) an expired copy wait of the stage kernel.
+static int check_waits(fe_domain* d) {
+  volatile int* f = d->waitErr;
+  if (!*f) return FE_OK;
+  *f = 0;
+  return set_err(FE_ERR_CUDA, "stage kernel: a wait for a tile copy expired");
+}
+
 extern "C" int fe_sync(fe_domain* d) {
   if (!d) return set_err(FE_ERR_ARG, "NULL handle");
   CU(cudaSetDevice(d->device));
   CU(cudaStreamSynchronize(d->stream));
   CU(cudaGetLastError());
+  if (int rc = check_waits(d)) return rc;
   if (d->mlp) return fe_mlp_check(d->mlp);
-  return FE_OK;
-}
-
-static int d2h(fe_domain* d, float* dst, const float* src, size_t nfloats) {
-  if (!dst) return FE_OK;
-  CU(cudaMemcpyAsync(dst, src, nfloats * sizeof(float), cudaMemcpyDeviceToHost, d->stream));
   return FE_OK;
 }
 
@@ -881,10 +1027,17 @@ extern "C" int fe_get_state(fe_domain* d, float* hydro, float* sgstke, float* mo
   CU(cudaSetDevice(d->device));
   const Phys& P = d->P;
   const size_t n = (size_t)P.n;
-  int rc = d2h(d, hydro, d->st[0], 5 * n);
-  if (!rc && P.ntke) rc = d2h(d, sgstke, d->st[0] + 5 * n, n);
-  if (!rc && P.nmoist) rc = d2h(d, moist, d->st[0] + (5 + P.ntke) * n, n * P.nmoist);
-  if (!rc) rc = d2h(d, pres, d->pr[0], n);
+  std::vector<FieldCopy> list;
+  add_fields(d, list, d->st[0], hydro, 5);
+  if (P.ntke) add_fields(d, list, d->st[0] + 5 * n, sgstke, 1);
+  if (P.nmoist) add_fields(d, list, d->st[0] + (5 + P.ntke) * n, moist, P.nmoist);
+  add_fields(d, list, d->pr[0], pres, 1);
+  if (pres) {
+    fe::k_pressure_level0<<<blocks1d(P.n2, 256), 256, 0, d->stream>>>(P, d->Q, d->st[0], d->pr[0]);
+    d->launches++;
+    CU(cudaGetLastError());
+  }
+  int rc = copy_fields(d, list, true);
   if (rc) return rc;
   CU(cudaStreamSynchronize(d->stream));
   return FE_OK;
@@ -915,7 +1068,7 @@ extern "C" int fe_build_frhs(fe_domain* d, int stage) {
   CU(cudaSetDevice(d->device));
   const Phys& P = d->P;
   if (!d->frhs) {
-    int rc = dev_alloc(d, &d->frhs, (size_t)P.n * P.nf);
+    int rc = dev_alloc_fields(d, &d->frhs, P.nf);
     if (rc) return rc;
   }
   float* A = d->st[0];
@@ -926,9 +1079,9 @@ extern "C" int fe_build_frhs(fe_domain* d, int stage) {
     CU(cudaGetLastError());
   }
   switch (stage) {
-    case 0: launch_stage<0, fe::MODE_FRHS>(d, d->stream, A, A, nullptr, d->pr[0], nullptr, d->frhs); break;
-    case 1: launch_stage<1, fe::MODE_FRHS>(d, d->stream, A, A, nullptr, d->pr[0], nullptr, d->frhs); break;
-    default: launch_stage<2, fe::MODE_FRHS>(d, d->stream, A, A, nullptr, d->pr[0], nullptr, d->frhs); break;
+    case 0: launch_stage<0, fe::MODE_FRHS>(d, d->stream, A, A, nullptr, d->pr[0], nullptr, field0(d->frhs)); break;
+    case 1: launch_stage<1, fe::MODE_FRHS>(d, d->stream, A, A, nullptr, d->pr[0], nullptr, field0(d->frhs)); break;
+    default: launch_stage<2, fe::MODE_FRHS>(d, d->stream, A, A, nullptr, d->pr[0], nullptr, field0(d->frhs)); break;
   }
   d->launches++;
   CU(cudaGetLastError());
@@ -942,10 +1095,13 @@ extern "C" int fe_get_frhs(fe_domain* d, float* hydroFrhs, float* sgstkeFrhs, fl
   CU(cudaSetDevice(d->device));
   const Phys& P = d->P;
   const size_t n = (size_t)P.n;
-  int rc = d2h(d, hydroFrhs, d->frhs, 5 * n);
-  if (!rc && P.ntke) rc = d2h(d, sgstkeFrhs, d->frhs + 5 * n, n);
-  if (!rc && P.nmoist) rc = d2h(d, moistFrhs, d->frhs + (5 + P.ntke) * n, n * P.nmoist);
-  if (!rc) rc = d2h(d, taus, d->Q.tau, 9 * n);
+  const float* F = field0(d->frhs);
+  std::vector<FieldCopy> list;
+  add_fields(d, list, F, hydroFrhs, 5);
+  if (P.ntke) add_fields(d, list, F + 5 * n, sgstkeFrhs, 1);
+  if (P.nmoist) add_fields(d, list, F + (5 + P.ntke) * n, moistFrhs, P.nmoist);
+  add_fields(d, list, d->Q.tau, taus, 9);
+  int rc = copy_fields(d, list, true);
   if (rc) return rc;
   CU(cudaStreamSynchronize(d->stream));
   return FE_OK;
@@ -961,12 +1117,13 @@ extern "C" int fe_get_sgs_fluxes(fe_domain* d, float* taus, float* moistTaus) {
   if (!d) return set_err(FE_ERR_ARG, "NULL handle");
   CU(cudaSetDevice(d->device));
   const Phys& P = d->P;
-  const size_t n = (size_t)P.n;
   if (taus && !P.turb) return set_err(FE_ERR_STATE, "no SGS stresses without turbulenceSelector");
   if (moistTaus && !(P.turb && P.nmoist > 0 && P.moistSGS > 0))
     return set_err(FE_ERR_STATE, "no moisture SGS fluxes in this configuration");
-  int rc = d2h(d, taus, d->Q.tau, 9 * n);
-  if (!rc) rc = d2h(d, moistTaus, d->Q.mtau, 3 * n * (size_t)P.nmoist);
+  std::vector<FieldCopy> list;
+  add_fields(d, list, d->Q.tau, taus, 9);
+  add_fields(d, list, d->Q.mtau, moistTaus, 3 * (size_t)P.nmoist);
+  int rc = copy_fields(d, list, true);
   if (rc) return rc;
   CU(cudaStreamSynchronize(d->stream));
   return FE_OK;
@@ -977,7 +1134,7 @@ extern "C" int fe_count_nonfinite(fe_domain* d, long long* count) {
   CU(cudaSetDevice(d->device));
   unsigned long long* dc = d->counter;
   cudaMemsetAsync(dc, 0, sizeof(unsigned long long), d->stream);
-  fe::k_nonfinite<<<blocks1d(d->P.n, 256), 256, 0, d->stream>>>(d->P, d->st[0], dc);
+  fe::k_nonfinite<<<blocks1d(d->P.nc, 256), 256, 0, d->stream>>>(d->P, d->st[0], dc);
   d->launches++;
   unsigned long long h = 0;
   cudaError_t e = cudaMemcpyAsync(&h, dc, sizeof(h), cudaMemcpyDeviceToHost, d->stream);
@@ -994,7 +1151,7 @@ extern "C" int fe_domain_means(fe_domain* d, double* means) {
   const int nf = d->P.nf;
   CU(cudaMalloc(&dm, sizeof(double) * nf));
   cudaMemsetAsync(dm, 0, sizeof(double) * nf, d->stream);
-  fe::k_means<<<blocks1d(d->P.n, 256), 256, 0, d->stream>>>(d->P, d->st[0], dm);
+  fe::k_means<<<blocks1d(d->P.nc, 256), 256, 0, d->stream>>>(d->P, d->st[0], dm);
   d->launches++;
   cudaError_t e = cudaMemcpyAsync(means, dm, sizeof(double) * nf, cudaMemcpyDeviceToHost, d->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(d->stream);
@@ -1020,11 +1177,14 @@ extern "C" int fe_set_stage_kernel(fe_domain* d, int kind, int tj, int ni) {
   if (!d) return set_err(FE_ERR_ARG, "NULL handle");
   if (kind != FE_KERNEL_CELL && kind != FE_KERNEL_MARCH) return set_err(FE_ERR_ARG, "unknown stage-kernel form");
   if (kind == FE_KERNEL_MARCH) {
+    const bool chosen = ni > 0;
     if (tj <= 0) tj = 8;
     if (ni <= 0) ni = d->mniDefault;
     if (tj != 4 && tj != 8) return set_err(FE_ERR_ARG, "march kernel: tj must be 4 or 8");
     d->mtj = tj;
     d->mni = ni;
+    const long long cols = (long long)((d->P.Nz + fe::MK - 1) / fe::MK) * ((d->P.Ny + tj - 1) / tj);
+    d->mniAuto = chosen ? 0 : march_planes(cols, d->P.Nx, (long long)(d->marchSlots) * 8 / tj);
   }
   d->kind = kind;
   invalidate_graph(d);
@@ -1085,7 +1245,7 @@ extern "C" int fe_autotune(fe_domain* d, int* tk, int* tj, int* ti) {
   struct Cand { int kind, a, b, c; };
   std::vector<Cand> cand;
   for (int tjm : {8, 4})
-    for (int ni : {16, 32, 64, 128, 256})
+    for (int ni : {2, 4, 8, 16, 32, 64})
       if (ni <= std::max(16, d->P.Nx)) cand.push_back({FE_KERNEL_MARCH, tjm, ni, 0});
   static const int cell[][3] = {{32, 4, 2}, {32, 8, 1}, {32, 2, 4}, {64, 2, 2}, {64, 4, 1}, {32, 4, 1}, {32, 2, 2}};
   for (auto& c : cell)
@@ -1097,6 +1257,7 @@ extern "C" int fe_autotune(fe_domain* d, int* tk, int* tj, int* ti) {
   size_t bi = 0;
   const int reps = 5;
   LocalImages local(d);
+  d->mniAuto = 0;  // the candidates' planes are the launched ones
   const int saved_kind = d->kind, saved_mtj = d->mtj, saved_mni = d->mni, saved_tk = d->tk, saved_tj = d->tj,
             saved_ti = d->ti;
   for (size_t c = 0; c < cand.size(); c++) {
@@ -1254,10 +1415,10 @@ extern "C" int fe_set_sgs_mlp(fe_domain* d, fe_mlp* m) {
   if (m && !d->P.turb) return set_err(FE_ERR_CONFIG, "the learned closure needs turbulenceSelector > 0");
   if (m && !d->feat) {
     CU(cudaSetDevice(d->device));
-    int rc = dev_alloc(d, &d->feat, (size_t)d->P.n * fe::SGS_NIN);
+    int rc = dev_alloc_fields(d, &d->feat, fe::SGS_NIN);
     if (rc) return rc;
   }
-  d->Q.feat = m ? d->feat : nullptr;
+  d->Q.feat = m ? field0(d->feat) : nullptr;
   d->mlp = m;
   invalidate_graph(d);
   return FE_OK;
@@ -1444,7 +1605,8 @@ static int ens_build_batch(fe_ensemble* e) {
   const size_t szM = sizeof(fe::MarchMember) * nm, szS = sizeof(fe::SgsMember) * nm;
   const size_t szF = sizeof(fe::SurfMember) * nm, szC = sizeof(fe::ClockMember) * nm;
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t total = 3 * (up(szM) + up(szS) + up(szF)) + up(szC) + up(4 * mB) + up(4 * sB) + up(4 * fB);
+  const size_t szT = sizeof(fe::MarchMaps) * nm;  // tensor maps (stages of 8-row tiles)
+  const size_t total = 3 * (up(szT) + up(szM) + up(szS) + up(szF)) + up(szC) + up(4 * mB) + up(4 * sB) + up(4 * fB);
   if (e->batchMem) cudaFree(e->batchMem);
   e->batchMem = nullptr;
   if (cudaMalloc(&e->batchMem, total) != cudaSuccess) {
@@ -1452,7 +1614,14 @@ static int ens_build_batch(fe_ensemble* e) {
     return set_err(FE_ERR_NOMEM, "ensemble table allocation failed");
   }
   char* p = (char*)e->batchMem;
+  std::vector<fe::MarchMaps> maps[3];
   for (int st = 0; st < 3; st++) {
+    for (int m = 0; m < nm; m++) {
+      maps[st].push_back(e->m[m]->maps[0][st]);
+      mm[st][m].maps = (const fe::MarchMaps*)p + m;
+    }
+    CU(cudaMemcpyAsync(p, maps[st].data(), szT, cudaMemcpyHostToDevice, e->stream));
+    p += up(szT);
     e->bMarch[st] = (fe::MarchMember*)p;
     CU(cudaMemcpyAsync(p, mm[st].data(), szM, cudaMemcpyHostToDevice, e->stream));
     p += up(szM);
@@ -1645,6 +1814,8 @@ extern "C" int fe_ensemble_sync(fe_ensemble* e) {
   CU(cudaStreamSynchronize(e->stream));
   for (auto* d : e->m) CU(cudaStreamSynchronize(d->stream));
   CU(cudaGetLastError());
+  for (auto* d : e->m)
+    if (int rc = check_waits(d)) return rc;
   return FE_OK;
 }
 

@@ -36,6 +36,24 @@ static __global__ void k_pbs(long long n, const float* __restrict__ thBS, float 
   if (t < n) pBS[t] = powf(thBS[t] * c1, cp_cv);
 }
 
+// Fields between the boundary's rows of nzh values and a domain's padded rows: one row of every
+// field of the list per warp.
+constexpr int PACK_MAX = 9;
+struct PackList {
+  float* p[PACK_MAX];
+};
+template <bool PACK>
+static __global__ void k_pack_rows(Phys P, PackList L, float* __restrict__ lin) {
+  const long long row = (long long)blockIdx.x * blockDim.y + threadIdx.y;
+  if (row >= (long long)P.nxh * P.nyh) return;
+  float* d = L.p[blockIdx.y] + row * P.sj;
+  float* h = lin + (long long)blockIdx.y * P.nc + row * P.nzh;
+  for (int k = threadIdx.x; k < P.nzh; k += 32) {
+    if (PACK) h[k] = d[k];
+    else d[k] = h[k];
+  }
+}
+
 // Source column of a halo column: its periodic image, or itself in a direction whose halos the
 // neighbouring slabs provide.
 __device__ __forceinline__ int wrap_i(const Phys& P, int i) {
@@ -49,11 +67,10 @@ __device__ __forceinline__ int wrap_j(const Phys& P, int j) {
 // the periodic source column, i.e. the reference's Commence BCs (cuda_hydroCoreDevice.cu:
 // 469-550) with every read of the current stage.
 static __global__ void k_fill(Phys P, Ptrs Q, float* st) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P.n) return;
-  const int k = (int)(t % P.nzh);
-  const int j = (int)((t / P.nzh) % P.nyh);
-  const int i = (int)(t / ((long long)P.nzh * P.nyh));
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= P.nc) return;
+  int i, j, k;
+  const long long c = cell_at(P, t, i, j, k);
   const bool inI = i >= P.iMin && i < P.iMax, inJ = j >= P.jMin && j < P.jMax, inK = k >= P.kMin && k < P.kMax;
   if (inI && inJ && inK) return;
   const int is = wrap_i(P, i), js = wrap_j(P, j);
@@ -73,20 +90,32 @@ static __global__ void k_fill(Phys P, Ptrs Q, float* st) {
       else if (f == 5 && P.ntke) v = below ? F[bot] : 0.0f;
       else v = below ? F[bot] : F[top];
     }
-    F[t] = v;
+    F[c] = v;
   }
 }
 
 // Perturbation pressure over the halo-inclusive block (cuda_pressureDevice.cu:53-113):
 // levels 1..kMin-1 use the kMin cell, levels >= kMax use kMax-1, level 0 its own cell.
 static __global__ void k_pressure(Phys P, Ptrs Q, const float* __restrict__ st, float* __restrict__ pres) {
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P.n) return;
-  const int k = (int)(t % P.nzh);
-  long long src = t;
-  if (k > 0 && k < P.kMin) src = t - k + P.kMin;
-  else if (k >= P.kMax) src = t - k + P.kMax - 1;
-  pres[t] = pert_pressure(P, st, Q.pBS, src);
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= P.nc) return;
+  int i, j, k;
+  const long long c = cell_at(P, t, i, j, k);
+  long long src = c;
+  if (k > 0 && k < P.kMin) src = c - k + P.kMin;
+  else if (k >= P.kMax) src = c - k + P.kMax - 1;
+  pres[c] = pert_pressure(P, st, Q.pBS, src);
+}
+
+// Perturbation pressure of level 0 of every column (level0_pressure of the column's periodic source).
+// No stencil reads it, so it is formed when the pressure is copied out, not in every commit.
+static __global__ void k_pressure_level0(Phys P, Ptrs Q, const float* __restrict__ st, float* __restrict__ pres) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)P.nxh * P.nyh) return;
+  const int i = (int)(t / P.nyh), j = (int)(t % P.nyh);
+  const long long s = (long long)wrap_i(P, i) * P.si + (long long)wrap_j(P, j) * P.sj;
+  const float qv = P.nmoist > 0 ? st[(long long)(5 + P.ntke) * P.n + s + P.kMin] : 0.0f;
+  pres[(long long)i * P.si + (long long)j * P.sj] = level0_pressure(P, Q, s, P.nmoist, qv);
 }
 
 // SGS length scale at cell c + dk (cuda_sgstkeDevice.cu:96-151), from primitives.
@@ -950,11 +979,10 @@ static __global__ void __launch_bounds__(256) k_stage(Phys P, Ptrs Q, const floa
   float pn;
   {
     float rtm = n4;
-    if (P.nmoist > 0) rtm = (float)((double)n4 * (1.0 + (double)(P.Rv_Rg * nq0 / n0) * 1e-3));
+    if (P.nmoist > 0) rtm = moist_rth(n4, __fdiv_rn(__fmul_rn(P.Rv_Rg, nq0), n0));
     pn = powf(rtm * P.c1, P.cp_cv) - Q.pBS[c];
   }
   store_images(P, pnxt, i, j, k, pn, atBot ? 2 : 0, atTop);
-  if (atBot) store_images(P, pnxt, i, j, 0, level0_pressure(P, Q, c - k, P.nmoist, nq0), 0, false);
 }
 
 static __global__ void k_clock(Ptrs Q, float dt) {
@@ -1008,12 +1036,11 @@ static __global__ void k_clock_list(const ClockMember* __restrict__ mem, int nme
 static __global__ void k_nonfinite(Phys P, const float* __restrict__ st, unsigned long long* out) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned int cnt = 0;
-  if (t < P.n) {
-    const int k = (int)(t % P.nzh);
-    const int j = (int)((t / P.nzh) % P.nyh);
-    const int i = (int)(t / ((long long)P.nzh * P.nyh));
+  if (t < P.nc) {
+    int i, j, k;
+    const long long c = cell_at(P, t, i, j, k);
     if (i >= P.iMin && i < P.iMax && j >= P.jMin && j < P.jMax && k >= P.kMin && k < P.kMax)
-      for (int f = 0; f < P.nf; f++) cnt += isfinite(st[(long long)f * P.n + t]) ? 0u : 1u;
+      for (int f = 0; f < P.nf; f++) cnt += isfinite(st[(long long)f * P.n + c]) ? 0u : 1u;
   }
   for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
   if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(out, (unsigned long long)cnt);
@@ -1039,7 +1066,7 @@ static __global__ void k_slab_partial(Phys P, Ptrs Q, const float* __restrict__ 
       const int i = (int)(col / P.nyh), j = (int)(col % P.nyh);
       const bool in = kin && i >= P.iMin && i < P.iMax && j >= P.jMin && j < P.jMax;
       const float* src = in ? cur : halo;
-      const long long c = col * P.nzh + k;
+      const long long c = (long long)i * P.si + (long long)j * P.sj + k;
       acc[0] += (double)src[c];
       acc[1] += (double)src[P.n + c];
       acc[2] += (double)src[2 * P.n + c];
@@ -1065,14 +1092,14 @@ static __global__ void k_slab_final(Phys P, Ptrs Q, int nblocks, int force) {
 static __global__ void k_means(Phys P, const float* __restrict__ st, double* out) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   bool in = false;
-  if (t < P.n) {
-    const int k = (int)(t % P.nzh);
-    const int j = (int)((t / P.nzh) % P.nyh);
-    const int i = (int)(t / ((long long)P.nzh * P.nyh));
+  long long c = 0;
+  if (t < P.nc) {
+    int i, j, k;
+    c = cell_at(P, t, i, j, k);
     in = i >= P.iMin && i < P.iMax && j >= P.jMin && j < P.jMax && k >= P.kMin && k < P.kMax;
   }
   for (int f = 0; f < P.nf; f++) {
-    double v = in ? (double)st[(long long)f * P.n + t] : 0.0;
+    double v = in ? (double)st[(long long)f * P.n + c] : 0.0;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&out[f], v);
   }

@@ -1,101 +1,91 @@
 // fe_march.cuh -- the fused stage kernel in i-marching form (sm_100a).
 //
-// A thread block owns a tile of 32 levels (k, one warp wide, so every row of the tile is one
-// 128-byte line) by TJ rows (j) and marches along i over a chunk of `ni` planes:
+// A thread block owns a tile of 32 levels (k) by TJ rows (j) and marches along i over a chunk of
+// `ni` planes. A thread computes two neighbouring levels of one row as the lanes of float2 values
+// (packed FP32: one instruction, two cells), 16 threads to a row. Within a plane the fields go two at
+// a time through one rolled loop: divergence, commit and stores of two fields. (Measured at 256x256x128,
+// second moist stage: every field unrolled 799 us, its instructions overflow the instruction cache,
+// stall "no instruction" 2.0 per issue; one field per iteration 719 us, more instructions.)
 //
-//   x direction   s(i..i+3) of every advected field live in registers (plus the prefetched
-//                 plane i+4), s(i-1) and s(i-2) are the thread's own cells of the two other
-//                 plane buffers; the x-face flux times the face velocity of the previous plane
-//                 is carried, so every x face is evaluated once.
-//   y, z          read a shared-memory copy of the (j,k) plane with a 3-cell ring. Three plane
-//                 buffers rotate: the thread's own value comes from its register window, the
-//                 ring of plane i+1 arrives by cp.async while plane i is computed, and one
-//                 __syncthreads per plane separates the two.
-//   face velocities  the contravariant velocities (D/rho)(m + w J) of plane i+1 are produced
-//                 one plane ahead into the same buffers (own cell plus a one-cell ring), so a
-//                 y or z face velocity costs one shared load.
-//   own-column inputs  s(i+4) of every field, p'(i+2), the metrics of plane i+2 and 1/D of
-//                 plane i+1 are copied by cp.async into a per-thread table one plane ahead, and
-//                 the carried x fluxes live in shared memory too: the registers hold only the
-//                 x window, so the 8-field flavour stays within 128 registers per thread.
+//   staging       tensor-map copies feed the loop. The ring planes of two fields (the (j,k) plane with
+//                 its 3-cell ring, for the y and z stencils) go through two stages that run ahead of
+//                 the loop; the tile's own cells (the x stencil) of planes i-2..i+3 stay in six
+//                 rotating slots per field. The last warp to finish a field pair of plane i refills
+//                 what it freed: the stage with the ring planes two pairs on, and the slots of plane
+//                 i-2 with the pair's plane i+4. Cells outside the array arrive as zeros.
+//   x direction   the x-face flux of the previous plane is carried (in shared memory), so every x face
+//                 is evaluated once
+//   HYB56         a face value is z0 plus five coefficients times first differences of the stencil
+//                 (hyb56_face); the coefficients depend on the face velocity's sign and b_hyb only,
+//                 so each face forms them once per plane for all fields, and the two faces of a
+//                 direction share their differences: 6 subtractions and 14 other operations for two
+//                 faces of two cells, where the flux in the reference's order takes 14 per face.
+//   face velocities  the contravariant velocities (D/rho)(m + w J) of plane i+1 are formed at the end
+//                 of plane i (own cells plus a one-cell ring) into two small planes, so a y or z face
+//                 velocity costs one shared load; one __syncthreads per plane.
 //
-// Everything else -- PGF, Rayleigh damping, buoyancy, Coriolis, SGS divergence and TKE budget,
-// saturation adjustment, the WS2002 commit with its halo images and the perturbation pressure
-// of the new state -- is the cell kernel's arithmetic (fe_kernels.cuh), term by term and in the
-// same order, evaluated on the register/shared copies.
+// The other terms -- PGF, Rayleigh damping, buoyancy, Coriolis, SGS tendencies, saturation
+// adjustment, the WS2002 commit with its halo images and the perturbation pressure of the new
+// state -- follow the cell kernel (fe_kernels.cuh). All arithmetic of a lane spells out its
+// roundings, so every instantiation gives the same bits for the same scheme and results do not
+// depend on the launch shape.
+//
+// What bounds it: latency. With 12 warps per SM (168 registers, 73 KB of shared memory per block of 128
+// threads) a warp issues every 6 to 7 cycles, issue slots 45 % busy, the FP32 pipe 28 %, DRAM below 25 %;
+// a block alone on an SM takes nearly as long per plane as beside two others. So what counts is the
+// length of a plane's instruction stream. Second stage of the moist hill at 256x256x128: 547 us, 1097
+// thread instructions per cell; one cell per thread with cp.async staging and a register window (16
+// warps) took 862 us and 2025 instructions. 512x512x128 with clouds: 2.05 ms.
 #pragma once
 #include "fe_kernels.cuh"
 #include "fe_march_launch.cuh"
+#include "fe_tma.cuh"
 
 namespace fe {
 
 constexpr int MK = 32;                      // levels per tile
-constexpr int MSLOTS = 9;                   // rho, rho u, rho v, rho w, rho theta, rho e, rho qv, rho ql, p'
-constexpr int SL_E = 5, SL_QV = 6, SL_QL = 7, SL_P = 8;
+constexpr int MT = MK / 2;                  // threads per row (two levels each)
+constexpr int SL_E = 5, SL_QV = 6, SL_QL = 7;   // roles of the fields after the five hydro fields
+constexpr int MRK = 40;                     // row pitch of a ring plane: levels k0-4..k0+35
 
-template <int TJ>
+constexpr int MSTG = 2;                     // ring-plane stages of two fields each
+
+// Shared-memory plan (floats) of a tile of TJ rows with room for NF fields.
+template <int TJ, int NF>
 struct MarchTile {
-  static constexpr int PJ = TJ + 6, PK = MK + 6;   // staged plane with a 3-cell ring
-  static constexpr int PLANE = PJ * PK;
-  static constexpr int CYN = (TJ + 2) * MK;        // contravariant y velocity, rows j = -1..TJ
-  static constexpr int CZK = MK + 2;               // contravariant z velocity, columns k = -1..MK
-  static constexpr int CZN = TJ * CZK;
-  static constexpr int BUF = MSLOTS * PLANE + CYN + CZN;
-  static constexpr int NT = MK * TJ;
-  static constexpr int RING = PLANE - TJ * MK;
-  static constexpr int RPT = (RING + NT - 1) / NT;  // ring cells per thread
-  static constexpr int CYT = 2 * MK, CZT = 2 * TJ;   // ring tasks of the velocity planes
-  static constexpr int NBUF = 3;
-  // per-thread tables: the inputs of the next plane (cp.async, double-buffered) and the
-  // carried x-face flux times velocity of every field
-  static constexpr int NAUX = 14;
-  static constexpr int AUX = 2 * NAUX * NT;
-  static constexpr int XC = 8 * NT;
-  static constexpr int SMEM_BYTES = (NBUF * BUF + AUX + XC) * 4;
+  static constexpr int NT = MT * TJ, NW = NT / 32;
+  static constexpr int OWNF = TJ * MK;                  // own cells of a field in a plane
+  static constexpr int OWN = NF * OWNF, NOWN = 6;
+  static constexpr int RINGF = (TJ + 6) * MRK;          // ring plane of a field: rows j0-3..j0+TJ+2
+  static constexpr int PRES = ((TJ + 2) * MRK + 31) / 32 * 32;   // p' plane: rows j0-1..j0+TJ
+  static constexpr int CYN = (TJ + 2) * MK;             // contravariant y velocity, rows -1..TJ
+  static constexpr int CZP = MK + 4;                    // pitch of the z velocity plane: level k at k+2
+  static constexpr int CZN = TJ * CZP;
+  static constexpr int STAGE = (2 * RINGF + 31) / 32 * 32;       // ring planes of a field pair
+  static constexpr int O_RING = NOWN * OWN, O_PRES = O_RING + MSTG * STAGE, O_VEL = O_PRES + PRES;
+  static constexpr int O_XC = O_VEL + 2 * (CYN + CZN);  // carried x fluxes [NF][NT] of float2
+  static constexpr int O_BAR = O_XC + NF * 2 * NT;      // mbarriers: MSTG stages, start; MSTG arrival counters
+  static_assert(O_RING % 32 == 0 && STAGE % 32 == 0 && O_PRES % 32 == 0 && O_XC % 32 == 0, "copy destinations on 128 bytes");
+  static_assert(O_VEL % 2 == 0 && O_XC % 2 == 0 && O_BAR % 2 == 0, "pairs and barriers on 8 bytes");
+  static constexpr int SMEM_BYTES = (O_BAR * 4 + (MSTG + 1) * 8 + MSTG * 4 + 15) / 16 * 16;
 };
-
-// Ring cell r of a staged plane: the 3 rows above and below the tile (full width), then the
-// 3 columns left and right of every tile row.
+// Fields a flavour has room for.
+template <int FL>
+__host__ __device__ constexpr int march_nf() {
+  return FL == FL_DRY ? 6 : 8;
+}
+template <int TJ, int FL>
+__host__ __device__ constexpr int march_smem_bytes() {
+  return MarchTile<TJ, march_nf<FL>()>::SMEM_BYTES;
+}
+// Thread blocks per SM: 12 warps (the 8-field tile of 8 rows takes 73 KB of the 227 KB, the registers
+// of 384 threads are 170 each).
 template <int TJ>
-__device__ __forceinline__ void march_ring_cell(int r, int& row, int& col) {
-  constexpr int PK = MK + 6;
-  if (r < 6 * PK) {
-    row = r / PK;
-    col = r - row * PK;
-    if (row >= 3) row += TJ;
-  } else {
-    const int q = r - 6 * PK;
-    row = 3 + q / 6;
-    const int cc = q - (q / 6) * 6;
-    col = cc < 3 ? cc : MK + cc;
-  }
+constexpr int march_blocks() {
+  return 384 / (MT * TJ);
 }
 
-__device__ __forceinline__ void cp_async4(float* sdst, const float* gsrc) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gsrc) : "memory");
-}
-// Pull the line holding p into L2 (no register, no wait). Only ever given addresses of cells
-// that exist in the array.
-__device__ __forceinline__ void prefetch_l2(const float* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-__device__ __forceinline__ bool slot_on(const Phys& P, int s) {
-  if (s < 5) return true;
-  if (s == SL_E) return P.ntke > 0;
-  if (s == SL_QV) return P.nmoist > 0;
-  if (s == SL_QL) return P.nmoist > 1;
-  return P.pgf != 0;
-}
-__device__ __forceinline__ const float* slot_src(const Phys& P, const float* cur, const float* pcur, int s) {
-  if (s < 5) return cur + (long long)s * P.n;
-  if (s == SL_E) return cur + 5LL * P.n;
-  if (s == SL_QV) return cur + (long long)(5 + P.ntke) * P.n;
-  if (s == SL_QL) return cur + (long long)(6 + P.ntke) * P.n;
-  return pcur;
-}
-// advection scheme of a slot as an ADV_* id (q_l's from moistureAdvSelectorQi)
+// advection scheme of a role as an ADV_* id (q_l's from moistureAdvSelectorQi) and its 1 - b
 __device__ __forceinline__ int slot_sel(const Phys& P, int s) {
   if (s < 5) return P.advSel;
   if (s == SL_E) return P.tkeAdvSel;
@@ -108,42 +98,11 @@ __device__ __forceinline__ float slot_b(const Phys& P, int s) {
   if (s == SL_QV) return P.qvB;
   return 0.0f;
 }
-
-// Compile-time configurations ("flavours") of the march kernel: fe_march_launch.cuh.
-template <int FL>
-__device__ __forceinline__ bool f_on(const Phys& P, int s) {
-  if constexpr (FL == FL_DRY) return s <= SL_E || s == SL_P;
-  else if constexpr (FL == FL_MOIST || FL == FL_MOIST34) return true;
-  else return slot_on(P, s);
-}
 template <int FL>
 __device__ __forceinline__ int f_sel(const Phys& P, int s) {
-  if constexpr (FL == FL_MOIST34) return s == SL_QL ? 5 : (s == SL_QV ? 2 : 3);
-  else if constexpr (FL != FL_ANY) return s == SL_QL ? 5 : 3;
+  if constexpr (FL == FL_MOIST34) return s == SL_QL ? ADV_WENO5 : (s == SL_QV ? ADV_HYB34 : ADV_HYB56);
+  else if constexpr (FL != FL_ANY) return s == SL_QL ? ADV_WENO5 : ADV_HYB56;
   else return slot_sel(P, s);
-}
-// Fields s and s + 1 (s even) evaluate their x faces as one lane pair: both present and on the
-// same scheme of the packed path, known at compile time. The moist flavours only: in the dry
-// flavour the pairs cost more registers than the 128 the launch shape allows (spills).
-template <int FL>
-__host__ __device__ constexpr bool x_paired(int s) {
-  if constexpr (FL == FL_ANY || FL == FL_DRY) {
-    return false;
-  } else {
-    if (s % 2 != 0 || s + 1 > SL_QL) return false;
-    const int a = FL == FL_MOIST34 ? (s == SL_QL ? 5 : (s == SL_QV ? 2 : 3)) : (s == SL_QL ? 5 : 3);
-    const int b = FL == FL_MOIST34 ? (s + 1 == SL_QL ? 5 : (s + 1 == SL_QV ? 2 : 3)) : (s + 1 == SL_QL ? 5 : 3);
-    return a == b && (a == ADV_HYB56 || a == ADV_WENO5);
-  }
-}
-template <int FL>
-__device__ __forceinline__ const float* f_src(const Phys& P, const float* cur, const float* pcur, int s) {
-  if constexpr (FL != FL_ANY) {
-    if (s == SL_P) return pcur;
-    return cur + (long long)s * P.n;  // slots 0..7 are fields 0..7 when TKE is prognostic
-  } else {
-    return slot_src(P, cur, pcur, s);
-  }
 }
 
 // SGS tendencies of the last-stage physics for the march kernel, one thread per interior cell
@@ -244,609 +203,671 @@ __global__ void __launch_bounds__(256, 4) k_sgs_tend(Phys P, Ptrs Q, const float
   for (int m = 1; m < NQ; m++) S[(5 + m) * n] = sq[m];
 }
 
+
+// ---------------------------------------------------------------- lane-pair helpers
+__device__ __forceinline__ float2 ld2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ void st2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
+// a * b by lanes, never contracted into a following addition (a packed product may be)
+__device__ __forceinline__ float2 prod2(float2 a, float2 b) { return f2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)); }
+__device__ __forceinline__ float2 rcp2(float2 a) { return f2(__frcp_rn(a.x), __frcp_rn(a.y)); }
+__device__ __forceinline__ float2 max2(float2 a, float b) { return f2(fmaxf(a.x, b), fmaxf(a.y, b)); }
+
+// Vertical halo copies of a committed pair at q: `nb` (2 or 3) levels below kMin repeat the first level,
+// the three levels above kMax-1 repeat the last one, which is lane x when topX.
+__device__ __forceinline__ void store_below(float* __restrict__ q, float v, int nb) {
+  st2(q - 2, f2s(v));
+  if (nb == 3) q[-3] = v;
+}
+__device__ __forceinline__ void store_above(float* __restrict__ q, float2 v, bool topX) {
+  float* t = q + (topX ? 1 : 2);
+  const float u = topX ? v.x : v.y;
+  t[0] = u; t[1] = u; t[2] = u;
+}
+
+// Saturation adjustment of a cell (cuda_moistureDevice.cu:80-247): the condensation rate; dth
+// receives the tendency it gives rho theta.
+__device__ __forceinline__ float sat_adjust(const Phys& P, const Ptrs& Q, long long c, float r0, float mth, float qv,
+                                            float ql, float& dth) {
+  const float ri = rinv(r0);
+  const float thd = mth * ri;
+  const float prd = P.condBasePres == 1 ? powf(Q.thBS[c] * P.c1, P.cp_cv) : powf(mth * P.c1, P.cp_cv);
+  const float Td = thd * powf(prd / P.p0, P.R_cp);
+  float pvs;
+  const float Tc = fmaxf(-80.0f, (Td - 273.16f));
+  if (Td >= 273.15f) {
+    pvs = (6.11239921f + Tc * (0.443987641f + Tc * (0.142986287e-1f + Tc * (0.264847430e-3f + Tc * (0.302950461e-5f +
+          Tc * (0.206739458e-7f + Tc * (0.640689451e-10f + Tc * (-0.952447341e-13f + -0.976195544e-15f * Tc)))))))) * 100.0f;
+  } else {
+    pvs = (6.11147274f + Tc * (0.503160820f + Tc * (0.188439774e-1f + Tc * (0.420895665e-3f + Tc * (0.615021634e-5f +
+          Tc * (0.602588177e-7f + Tc * (0.385852041e-9f + Tc * (0.146898966e-11f + 0.252751365e-14f * Tc)))))))) * 100.0f;
+  }
+  pvs = fminf((0.99f * prd), pvs);
+  float ffor = 0.0f;
+  const float flim = ql * 1e-3f;
+  if (P.moistCond == 1) {
+    ffor = qv * 1e-3f - (pvs / (P.R_vapor * Td));
+  } else if (P.moistCond == 2) {
+    const float rv = qv * 1e-3f, rvs = pvs / (P.R_vapor * Td);
+    ffor = (rv - rvs) / (1.0f + (powf(P.L_v, 2.0f) * rvs * ri / (P.cp_gas * P.R_vapor * powf(Td, 2.0f))));
+  } else {
+    const float rv = qv * 1e-3f;
+    float rvs = pvs / (prd - pvs) / P.Rv_Rg;
+    rvs = rvs / ri;
+    ffor = (rv - rvs) / (1.0f + (powf(P.L_v, 2.0f) * rvs * ri / (P.cp_gas * P.R_vapor * powf(Td, 2.0f))));
+  }
+  float fc = fmaxf(ffor, 0.0f) - fmaxf(fminf(flim, -ffor), 0.0f);
+  fc = fc / P.condTscale;
+  const float prd2 = powf(mth * P.c1, P.cp_cv);
+  const float Td2 = thd * powf(prd2 / P.p0, P.R_cp);
+  dth = ((thd * P.L_v) / (Td2 * P.cp_gas)) * fc;
+  return fc;
+}
+
+// Rayleigh damping of rho w in the sponge layer added to F.
+__device__ __forceinline__ float rayleigh(const Phys& P, float F, float z, float zt, float r0, float w) {
+  if (!(z >= (zt - P.dampDepth))) return F;
+  const float pio2 = 1.5707963267948966f;
+  const double sn = (double)sinf((float)((double)pio2 * (1.0 - (double)((zt - z) / P.dampDepth))));
+  return (float)((double)F - 0.2 * (double)r0 * (sn * sn) * (double)__fmul_rn(w, __frcp_rn(r0)));
+}
+
 // MP: the saturation adjustment of the last stage. -1 decides per step from the device clock;
 // 0 and 1 are the two halves of a pair launched back to back, each returning at once unless the
 // step is its kind (0: no adjustment this step, compiled without the adjustment; 1: adjustment).
 // The body of one thread block: tile (bx, by, bz) of the domain P / Q (k tile, j tile, i chunk).
 template <int STAGE, int MODE, int TJ, int FL, int MP>
-__device__ __forceinline__ void march_body(const Phys& P, const Ptrs& Q, const float* __restrict__ cur,
-                                           const float* __restrict__ base, float* __restrict__ nxt,
-                                           const float* __restrict__ pcur, float* __restrict__ pnxt,
-                                           float* __restrict__ frhs, int ni, int bx, int by, int bz) {
-  const int ntke = FL == FL_ANY ? P.ntke : 1;
-  const int nmoist = FL == FL_ANY ? P.nmoist : ((FL == FL_MOIST || FL == FL_MOIST34) ? 2 : 0);
-  const bool pgf = FL == FL_ANY ? (P.pgf != 0) : true;
-  const bool tke = FL == FL_ANY ? (P.tke != 0) : true;
+__device__ __forceinline__ void march_body(const Phys& P, const Ptrs& Q, const MarchMaps* __restrict__ maps,
+                                           const float* __restrict__ cur, const float* __restrict__ base,
+                                           float* __restrict__ nxt, const float* __restrict__ pcur,
+                                           float* __restrict__ pnxt, float* __restrict__ frhs, int ni, int bx, int by,
+                                           int bz) {
+  constexpr bool ANY = FL == FL_ANY;
+  constexpr int NF = march_nf<FL>();
+  using T = MarchTile<TJ, NF>;
+  const int nf = ANY ? P.nf : NF;
+  const int ntke = ANY ? P.ntke : 1;
+  const int nmoist = ANY ? P.nmoist : ((FL == FL_MOIST || FL == FL_MOIST34) ? 2 : 0);
+  const bool pgf = ANY ? (P.pgf != 0) : true;
+  const bool tke = ANY ? (P.tke != 0) : true;
   // physics stages: every stage without oneRK, else the last; the flavours fix oneRK = 1
-  const bool phys = FL == FL_ANY ? ((P.oneRK == 0) || (STAGE == 2)) : (STAGE == 2);
+  const bool phys = ANY ? ((P.oneRK == 0) || (STAGE == 2)) : (STAGE == 2);
   const bool mpNow = phys && nmoist > 1 && P.moist && P.moistCond > 0 && ((*Q.clockIt) % P.mpFreq == 0);
   if ((MP == 0 && mpNow) || (MP == 1 && !mpNow)) return;  // the other half of the pair runs this step
   const bool mpStep = MP == 0 ? false : mpNow;
   // large-scale forcing inline only without the SGS kernel (which otherwise carries it)
-  const bool lsfNow = STAGE == 2 && FL == FL_ANY && !P.turb && lsf_step(P, *Q.clockIt);
-  using T = MarchTile<TJ>;
-  constexpr int PK = T::PK, PLANE = T::PLANE;
-  extern __shared__ __align__(16) float sm[];
+  const bool lsfNow = STAGE == 2 && ANY && !P.turb && lsf_step(P, *Q.clockIt);
+  constexpr bool same = STAGE == 0;  // the first stage's commit base is its input state
 
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * MK + tx;
+  extern __shared__ __align__(1024) float sm[];
+  uint64_t* const bar = reinterpret_cast<uint64_t*>(sm + T::O_BAR);        // [MSTG] stages, then the start
+  unsigned* const cnt = reinterpret_cast<unsigned*>(bar + MSTG + 1);       // [MSTG] warps done with a stage
+
+  if (tma_smem(sm) & 127u) {  // tensor-map copies need their destinations on 128 bytes
+    if (Q.waitErr) *Q.waitErr = 1;
+    return;
+  }
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * MT + tx;
   const int k0 = P.kMin + bx * MK, j0 = P.jMin + by * TJ;
   const int i0 = P.iMin + bz * ni;
   const int i1 = min(i0 + ni, P.iMax);
-  const int k = k0 + tx, j = j0 + ty;
-  const bool inArr = (k < P.nzh) && (j < P.nyh);     // the thread's column exists in memory
-  const bool active = (k < P.kMax) && (j < P.jMax);  // ... and is an interior column
+  const int k = k0 + 2 * tx, j = j0 + ty;            // lane x is level k, lane y level k + 1
+  const bool inArr = (k < P.nzh) && (j < P.nyh);     // the pair exists in memory
+  const bool active = (k < P.kMax) && (j < P.jMax);  // ... and holds an interior cell
+  const bool both = k + 1 < P.kMax;                  // ... two of them
   const long long n = P.n;
   const int si = P.si, sj = P.sj;
-  const long long col = (long long)j * sj + k;
-  const long long tile0 = (long long)j0 * sj + k0;
-  const int own = (ty + 3) * PK + (tx + 3);
+  // byte offset of the pair within a plane; threads outside the array read the tile's first pair instead
+  const unsigned colB = (unsigned)(inArr ? j * sj + k : j0 * sj + k0) * 4u;
   const float dXi = P.dXi, dYi = P.dYi, dZi = P.dZi;
+  const int own = ty * MK + 2 * tx;                          // the pair in an own-cell plane of a field
+  const int rng = (ty + 3) * MRK + (2 * tx + 4);             // ... in a ring plane
+  const int prs = (ty + 1) * MRK + (2 * tx + 4);             // ... in the p' plane
+  // the pair of a field of a plane starting at `ub` (uniform): uniform base plus 32-bit offset
+  auto g2 = [&](const float* ub) -> float2 {
+    return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(ub) + colB);
+  };
+  auto role_of = [&](int f) -> int { return ANY ? (f < 5 ? f : (f == 5 && ntke ? SL_E : f - 5 - ntke + SL_QV)) : f; };
 
-  // ring cells of the staged planes handled by this thread
-  int rS[T::RPT], rG[T::RPT];
-  bool rV[T::RPT], rN[T::RPT];
-#pragma unroll
-  for (int q = 0; q < T::RPT; q++) {
-    const int r = tid + q * T::NT;
-    rV[q] = false; rN[q] = false; rS[q] = 0; rG[q] = 0;
-    if (r < T::RING) {
-      int row, cl;
-      march_ring_cell<TJ>(r, row, cl);
-      const int jj = j0 + row - 3, kk = k0 + cl - 3;
-      rV[q] = (jj < P.nyh) && (kk < P.nzh);
-      rN[q] = row >= 2 && row <= TJ + 3 && cl >= 2 && cl <= MK + 3;  // within one cell (p' ring)
-      rS[q] = row * PK + cl;
-      rG[q] = (row - 3) * sj + (cl - 3);
-    }
-  }
-  // velocity-plane ring task: cy at rows -1 and TJ, or cz at columns -1 and MK
+  // velocity-plane ring task: cy at rows -1 and TJ (pairs), or cz at columns -1 and MK (one cell).
+  // Its inputs of plane ip are loaded ahead, its velocity stored with the own cells'.
   int rtKind = 0, rtS = 0;
-  long long rtOff = 0;
+  unsigned rtB = 0;
   {
     int row = 0, cc = 0;
-    if (tid < T::CYT) {
-      rtKind = 1; row = (tid < MK) ? -1 : TJ; cc = tid & (MK - 1);
+    if (tid < 2 * MT) {
+      rtKind = 1; row = (tid < MT) ? -1 : TJ; cc = 2 * (tid & (MT - 1));
       rtS = (row + 1) * MK + cc;
-    } else if (tid < T::CYT + T::CZT) {
-      const int q = tid - T::CYT;
+    } else if (tid < 2 * MT + 2 * TJ) {
+      const int q = tid - 2 * MT;
       rtKind = 2; row = q >> 1; cc = (q & 1) ? MK : -1;
-      rtS = T::CYN + row * T::CZK + (cc + 1);
+      rtS = T::CYN + row * T::CZP + (cc + 2);
     }
     const int jj = j0 + row, kk = k0 + cc;
     if (rtKind && !(jj < P.nyh && kk < P.nzh)) rtKind = 0;
-    rtOff = (long long)jj * sj + kk;
+    rtB = (unsigned)(jj * sj + kk) * 4u;
   }
-
-  auto issue_ring = [&](int ip, float* buf) {
-    const long long pl = (long long)ip * si + tile0;
-#pragma unroll
-    for (int s = 0; s < MSLOTS; s++) {
-      if (!f_on<FL>(P, s)) continue;
-      const float* src = f_src<FL>(P, cur, pcur, s) + pl;
-#pragma unroll
-      for (int q = 0; q < T::RPT; q++)
-        if (rV[q] && (s != SL_P || rN[q])) cp_async4(buf + s * PLANE + rS[q], src + rG[q]);
+  float2 tD = f2s(0.0f), tJ = tD, tR = f2s(1.0f), tM = tD, tW = tD;
+  auto task_load = [&](int ip) {
+    const long long po = (long long)ip * si;
+    if (rtKind == 1) {
+      auto at = [&](const float* ub) { return *reinterpret_cast<const float2*>(reinterpret_cast<const char*>(ub + po) + rtB); };
+      tD = at(Q.D); tJ = at(Q.J32); tR = at(cur); tM = at(cur + 2 * n); tW = at(cur + 3 * n);
+    } else if (rtKind == 2) {
+      auto at = [&](const float* ub) { return *reinterpret_cast<const float*>(reinterpret_cast<const char*>(ub + po) + rtB); };
+      tD.x = at(Q.D); tJ.x = at(Q.J33); tR.x = at(cur); tW.x = at(cur + 3 * n);
     }
-    cp_async_commit();
+  };
+  auto task_store = [&](float* vel) {
+    if (rtKind == 1) st2(vel + rtS, f2(contra(tD.x, tR.x, tM.x, tW.x, tJ.x), contra(tD.y, tR.y, tM.y, tW.y, tJ.y)));
+    else if (rtKind == 2) vel[rtS] = contra_z(tD.x, tR.x, tW.x, tJ.x);
+  };
+
+  float* const presB = sm + T::O_PRES;
+  auto velB = [&](int q) -> float* { return sm + T::O_VEL + q * (T::CYN + T::CZN); };
+  float2* const xcs = reinterpret_cast<float2*>(sm + T::O_XC) + tid;  // [NF][NT]
+  const int xk = k0 + ROW_PAD;                                        // the tile's first level in a padded row
+  constexpr uint32_t ringBytes = 2 * T::RINGF * 4, ownBytes = 2 * T::OWNF * 4, presBytes = (TJ + 2) * MRK * 4;
+  bool dead = false;  // a wait expired: finish without further waits (no access depends on the data)
+  auto wait = [&](int s, uint32_t phase) {
+    if (!dead && !tma_bar_wait(bar + s, phase)) {
+      dead = true;
+      if (Q.waitErr) *Q.waitErr = 1;
+    }
   };
 
   // ---------------------------------------------------------------- prologue (plane i0)
-  // buffers: plane i0 -> 0, plane i0+1 -> 1 (holds s(i0-2) at the own cell until it is
-  // refilled), plane i0-1 -> 2
-  float w[8][4];
-  float pc1 = 0.0f;   // p'(i+1)
-  float Dc = 0.0f, Dn = 0.0f, J1c = 0.0f, J1n = 0.0f, J2c = 0.0f, J3c = 0.0f;
-  const long long cA = (long long)i0 * si + col;
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-#pragma unroll
-    for (int d = 0; d < 4; d++) w[s][d] = 0.0f;
-  }
-  float* const B0 = sm;
-  float* const B1 = sm + T::BUF;
-  float* const B2 = sm + 2 * T::BUF;
-  float* const aux = sm + T::NBUF * T::BUF;   // [2][NAUX][NT]
-  float* const xcs = aux + T::AUX;            // [8][NT]
-  // the inputs of step ib+1 (loaded during step ib): slots 0..7 s(ib+4), 8 p'(ib+2), 9 D(ib+2),
-  // 10 J31(ib+2), 11 J32(ib+2), 12 J33(ib+2), 13 invD(ib+1)
-  auto issue_aux = [&](int ib, float* tbl) {
-    float* const buf = tbl + tid;  // this thread's entry of each slot
-    const long long c = (long long)ib * si + col;
-    if (inArr) {
-      if (ib + 4 < P.nxh) {
-#pragma unroll
-        for (int s = 0; s < 8; s++)
-          if (f_on<FL>(P, s)) cp_async4(buf + s * T::NT, f_src<FL>(P, cur, pcur, s) + c + 4 * (long long)si);
-      }
-      if (pgf) cp_async4(buf + 8 * T::NT, pcur + c + 2 * (long long)si);
-      cp_async4(buf + 9 * T::NT, Q.D + c + 2 * (long long)si);
-      cp_async4(buf + 10 * T::NT, Q.J31 + c + 2 * (long long)si);
-      cp_async4(buf + 11 * T::NT, Q.J32 + c + 2 * (long long)si);
-      cp_async4(buf + 12 * T::NT, Q.J33 + c + 2 * (long long)si);
-      cp_async4(buf + 13 * T::NT, Q.invD + c + si);
+  // own-cell slots: plane q is in slot (q - i0 + 2) % 6; slots 0..5 start as planes i0-2 .. i0+3
+  if (tid == 0) {
+    for (int s = 0; s <= MSTG; s++) tma_bar_init(bar + s);
+    for (int s = 0; s < MSTG; s++) cnt[s] = 0;
+    tma_bar_expect(bar + MSTG, 7u * nf * T::OWNF * 4 + (pgf ? presBytes : 0));
+    for (int q = 0; q < 6; q++) tma_load4(sm + q * T::OWN, &maps->ownAll, xk, j0, i0 - 2 + q, 0, bar + MSTG);
+    // plane i0-3, read once below, lands where the carried x fluxes go (the same layout)
+    tma_load4(sm + T::O_XC, &maps->ownAll, xk, j0, i0 - 3, 0, bar + MSTG);
+    if (pgf) tma_load3(presB, &maps->pres, xk - 4, j0 - 1, i0, bar + MSTG);
+    for (int s = 0; s < MSTG; s++) {
+      tma_bar_expect(bar + s, ringBytes);
+      tma_load4(sm + T::O_RING + s * T::STAGE, &maps->ring, xk - 4, j0 - 3, i0, 2 * s, bar + s);
     }
-    cp_async_commit();
+  }
+  __syncthreads();
+  float2 J1 = f2s(0.0f), J2 = J1, J3 = J1, iD = J1;              // metrics of plane i
+  float2 nD = J1, nJ1 = J1, nJ2 = J1, nJ3 = J1, niD = J1;        // ... of plane i + 1
+  float2 pm = J1, p0 = J1, pp = J1;                               // own p' of planes i-1, i, i+1
+  float2 cx0;
+  {
+    const long long po = (long long)i0 * si;
+    const float2 Dm = g2(Q.D + po - si), J1m = g2(Q.J31 + po - si), D0 = g2(Q.D + po);
+    J1 = g2(Q.J31 + po); J2 = g2(Q.J32 + po); J3 = g2(Q.J33 + po); iD = g2(Q.invD + po);
+    nD = g2(Q.D + po + si); nJ1 = g2(Q.J31 + po + si); nJ2 = g2(Q.J32 + po + si); nJ3 = g2(Q.J33 + po + si);
+    niD = g2(Q.invD + po + si);
+    if (pgf) { pm = g2(pcur + po - si); p0 = g2(pcur + po); pp = g2(pcur + po + si); }
+    task_load(i0);
+    wait(MSTG, 0);
+    const float *oM2 = sm + own, *oM1 = oM2 + T::OWN, *o0 = oM1 + T::OWN, *oP1 = o0 + T::OWN, *oP2 = oP1 + T::OWN;
+    const float2 drm = f2(__fdiv_rn(Dm.x, oM1[0]), __fdiv_rn(Dm.y, oM1[1]));
+    const float2 dr0 = f2(__fdiv_rn(D0.x, o0[0]), __fdiv_rn(D0.y, o0[1]));
+    const float2 w0 = ld2(o0 + 3 * T::OWNF);
+    const float2 cxm = prod2(drm, fma2(ld2(oM1 + 3 * T::OWNF), J1m, ld2(oM1 + T::OWNF)));
+    cx0 = prod2(dr0, fma2(w0, J1, ld2(o0 + T::OWNF)));
+    const float2 cyO = prod2(dr0, fma2(w0, J2, ld2(o0 + 2 * T::OWNF))), czO = prod2(dr0, prod2(w0, J3));
+    const float2 um = mul2(f2s(0.5f * dXi), add2(cx0, cxm));  // velocity of the face i0-1/2
+#pragma unroll 1
+    for (int f = 0; f < nf; f++) {
+      const int role = role_of(f);
+      const int sel = f_sel<FL>(P, role), o = f * T::OWNF;
+      const float bf = 1.0f - slot_b(P, role);
+      const float2 m3 = xcs[f * T::NT];
+      const float2 m2 = ld2(oM2 + o), m1 = ld2(oM1 + o), z0 = ld2(o0 + o), q1 = ld2(oP1 + o), q2 = ld2(oP2 + o);
+      float2 fx;
+      if (sel == ADV_HYB56)
+        fx = hyb56_face(hyb56_coef(um, bf), m1, dif2(z0, m1), dif2(q1, z0), dif2(q2, q1), dif2(m1, m2), dif2(m2, m3));
+      else
+        fx = adv_face2<true>(sel, m3, m2, m1, z0, q1, q2, um, f2s(bf));
+      xcs[f * T::NT] = mul2(um, fx);
+    }
+    float* v = velB(0);
+    st2(v + (ty + 1) * MK + 2 * tx, cyO);
+    st2(v + T::CYN + ty * T::CZP + 2 * tx + 2, czO);
+    task_store(v);
+  }
+  __syncthreads();
+  // base density and height of the plane's pair, and the height of the column's last level
+  float2 rbs = f2s(0.0f), z = rbs;
+  float zt = 0.0f;
+  auto load_base = [&](int ip) {
+    const long long pq = (long long)ip * si;
+    if (P.buoy) rbs = g2(Q.rhoBS + pq);
+    if (P.cor || P.damp) z = g2(Q.zPos + pq);
+    if (P.damp && inArr) zt = Q.zPos[pq + (long long)j * sj + (P.kMax - 1)];
   };
-  if (!inArr) {
-    for (int q = 0; q < 2 * T::NAUX; q++) aux[q * T::NT + tid] = 0.0f;
-    for (int q = 0; q < 8; q++) xcs[q * T::NT + tid] = 0.0f;
-  }
-  issue_aux(i0 - 1, aux + T::NAUX * T::NT);  // read by step i0 (buffer 1)
-  float Dm1 = 0.0f, J1m1 = 0.0f, rm1 = 0.0f, um1 = 0.0f, wm1 = 0.0f, p0v = 0.0f, pm1 = 0.0f;
-  if (inArr) {
-    Dm1 = Q.D[cA - si]; Dc = Q.D[cA];
-    J1m1 = Q.J31[cA - si]; J1c = Q.J31[cA];
-    J2c = Q.J32[cA]; J3c = Q.J33[cA];
-    if (pgf) { pm1 = pcur[cA - si]; p0v = pcur[cA]; }
-  }
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    if (!f_on<FL>(P, s)) continue;
-    const float* src = f_src<FL>(P, cur, pcur, s);
-    float sm2 = 0.0f, sm1 = 0.0f;
-    if (inArr) {
-      sm2 = src[cA - 2 * (long long)si]; sm1 = src[cA - si];
-#pragma unroll
-      for (int d = 0; d < 3; d++) w[s][d] = src[cA + d * (long long)si];
-    }
-    B1[s * PLANE + own] = sm2;
-    B2[s * PLANE + own] = sm1;
-    B0[s * PLANE + own] = w[s][0];
-    if (s == 0) rm1 = sm1;
-    if (s == 1) um1 = sm1;
-    if (s == 3) wm1 = sm1;
-  }
-  if (pgf) { B0[SL_P * PLANE + own] = p0v; B2[SL_P * PLANE + own] = pm1; }
-  float cx0 = contra(Dc, w[0][0], w[1][0], w[3][0], J1c);
-  float upPrev;
-  {
-    const float cxm = contra(Dm1, rm1, um1, wm1, J1m1);
-    upPrev = (0.5f * dXi) * (cx0 + cxm);  // velocity of the face i0-1/2
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-      if (!f_on<FL>(P, s)) continue;
-      const float* src = f_src<FL>(P, cur, pcur, s);
-      const float m3 = inArr ? src[cA - 3 * (long long)si] : 0.0f;
-      const float m2 = B1[s * PLANE + own], m1 = B2[s * PLANE + own];
-      const float f = adv_face<true>(f_sel<FL>(P, s), m3, m2, m1, w[s][0], w[s][1], w[s][2], upPrev, 1.0f - slot_b(P, s));
-      xcs[s * T::NT + tid] = __fmul_rn(upPrev, f);
-    }
-  }
-  float cyOwn, czOwn;
-  {
-    issue_ring(i0, B0);
-    cyOwn = contra(Dc, w[0][0], w[2][0], w[3][0], J2c);
-    czOwn = contra_z(Dc, w[0][0], w[3][0], J3c);
-    float* v = B0 + MSLOTS * PLANE;
-    v[(ty + 1) * MK + tx] = cyOwn;
-    v[T::CYN + ty * T::CZK + tx + 1] = czOwn;
-    if (rtKind) {
-      const long long c = (long long)i0 * si + rtOff;
-      const float D = Q.D[c], r = cur[c];
-      v[rtS] = rtKind == 1 ? contra(D, r, cur[2 * n + c], cur[3 * n + c], Q.J32[c]) : contra_z(D, r, cur[3 * n + c], Q.J33[c]);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-  }
+  load_base(i0);
+  // slots of planes i-2 .. i+3 (float offsets)
+  int sM2 = 0, sM1 = T::OWN, s0 = 2 * T::OWN, sP1 = 3 * T::OWN, sP2 = 4 * T::OWN, sP3 = 5 * T::OWN;
+  int stg = 0;            // stage and parity of the loop's next ring plane
+  uint32_t par = 0;
 
-  const bool same = (base == cur);  // first stage: the commit base is the input state
+  // WS2002 RK3 commit (cuda_RKschemes.cu:113-157). Stage 1's factor dt/3 is not a float: its low part
+  // is added too, so the increment keeps the double product's accuracy; stage 2's dt/2 and stage
+  // 3's dt are floats, whose fused product is exact.
+  const double cd = STAGE == 0 ? (1.0 / 3.0) * (double)P.dt : (STAGE == 1 ? 0.5 * (double)P.dt : (double)P.dt);
+  const float chi = (float)cd, clo = (float)(cd - (double)chi);
+  const float kq = 1e-3f, kqLo = (float)(1e-3 - (double)kq);  // g/kg: 1e-3 as a float and its remainder
+  const bool topX = k == P.kMax - 1;
+  const bool atBot = (k == P.kMin), atTop = active && (topX || k + 1 == P.kMax - 1);
+  const bool jlo = j < P.jMin + 3, jhi = j >= P.jMax - 3;
+  const bool pairOut = active && both, oneOut = active && !both;         // the pair's cells to commit
+  const bool botOut = active && atBot, topOut = active && atTop;         // ... and their vertical halo copies
+  // fields that take an SGS tendency in this stage (bit f: field f - 1 of the SGS kernel's seven)
+  unsigned sgsMask = 0;
+  if (phys && P.turb) {
+    for (int f = 1; f < nf; f++) {
+      const int role = role_of(f);
+      if (role < 5 || (role == SL_E && tke) || (role == SL_QV && (P.moistSGS > 0 || P.lsf)) || (role == SL_QL && P.moistSGS > 0))
+        sgsMask |= 1u << f;
+    }
+  }
+  const bool filt = P.filt != 0, keepF = MODE == MODE_FRHS || (STAGE == 2 && frhs);
 
   // ---------------------------------------------------------------- march
-  float *cs = B0, *ns = B1, *ps = B2;  // planes i, i+1 (own cell: s(i-2) until refilled), i-1
   for (int i = i0; i < i1; i++) {
     const bool more = (i + 1 < i1);
-    const long long c = (long long)i * si + col;
+    const int b = (i - i0) & 1;
+    const long long po = (long long)i * si;
+    if (tid == 0 && more) {
+      // what later planes load straight from memory, into L2: the next plane's commit base, SGS
+      // tendencies and base state, the metrics and p' two planes ahead
+      if (MODE != MODE_FRHS && !same) tma_prefetch4(&maps->base, xk, j0, i + 1, 0);
+      if (phys && P.turb) tma_prefetch4(&maps->sgs, xk, j0, i + 1, 0);
+      if (MODE != MODE_FRHS) tma_prefetch4(&maps->bs, xk, j0, i + 1, 2);
+      if (P.buoy) tma_prefetch4(&maps->bs, xk, j0, i + 1, 0);
+      tma_prefetch4(&maps->grid, xk, j0, i + 2, 0);
+      if (pgf) tma_prefetch3(&maps->pres, xk - 4, j0 - 1, i + 2);
+    }
+    const float* const own0 = sm + s0 + own;   // own cells of plane i, field f at f * OWNF
+    const float* const own1 = sm + sP1 + own;  // ... of plane i + 1
 
-    // this plane's table (loaded during the previous step): the new end of the x window and the
-    // metrics of plane i+1; then start the next one
-    const float* ax = aux + ((i - i0 + 1) & 1) * T::NAUX * T::NT + tid;
-#pragma unroll
-    for (int s = 0; s < 8; s++)
-      if (f_on<FL>(P, s)) w[s][3] = ax[s * T::NT];
-    if (pgf) pc1 = ax[8 * T::NT];
-    Dn = ax[9 * T::NT];
-    J1n = ax[10 * T::NT];
-    // the next plane's single-cell reads (commit base, base state, SGS fields written by the
-    // physics kernel) into L2 while this plane is computed
-    if (more && active) {
-      const long long cn = c + si;
-      if (MODE != MODE_FRHS && !same) {
-#pragma unroll
-        for (int s = 0; s < 8; s++)
-          if (f_on<FL>(P, s)) prefetch_l2(f_src<FL>(P, base, pcur, s) + cn);
-      }
-      if (MODE != MODE_FRHS) prefetch_l2(Q.pBS + cn);
-      if (P.buoy || P.cor || P.damp) prefetch_l2(Q.rhoBS + cn);
-      if (P.cor || P.damp) prefetch_l2(Q.zPos + cn);
-      if (phys && P.turb) {
-#pragma unroll
-        for (int m = 0; m < 5; m++) prefetch_l2(Q.sgsF + m * n + cn);
-        if (nmoist > 0 && P.moistSGS > 0)
-          for (int m = 0; m < nmoist; m++) prefetch_l2(Q.sgsF + (5 + m) * n + cn);
-      }
-    }
-    // inputs of this plane's commit, loaded before the advection so that their memory latency
-    // overlaps it (and before any store of the plane: the stores may alias `base`)
-    float cb[8];
-    float pbs = 0.0f;
-#pragma unroll
-    for (int s = 0; s < 8; s++) cb[s] = 0.0f;
-    if (MODE != MODE_FRHS && active) {
-#pragma unroll
-      for (int s = 0; s < 8; s++)
-        if (f_on<FL>(P, s) && !same) cb[s] = f_src<FL>(P, base, pcur, s)[c];
-      pbs = Q.pBS[c];
-    }
-    // SGS tendencies of this cell (k_sgs_tend): stress divergence on rho u, rho v, rho w, heat
-    // flux divergence, the TKE budget, moisture flux divergences
-    float sg[7];
-#pragma unroll
-    for (int m = 0; m < 7; m++) sg[m] = 0.0f;
-    if (phys && P.turb && active) {
-#pragma unroll
-      for (int m = 0; m < 4; m++) sg[m] = Q.sgsF[m * n + c];
-      if (tke) sg[4] = Q.sgsF[4 * n + c];
-      if (nmoist > 0 && (P.moistSGS > 0 || P.lsf)) {
-        sg[5] = Q.sgsF[5 * n + c];
-        if (nmoist > 1 && P.moistSGS > 0) sg[6] = Q.sgsF[6 * n + c];
-      }
-    }
-    // base state of the buoyancy, Rayleigh and Coriolis terms
-    float zc = 0.0f, ztop = 0.0f, rbsc = 0.0f;
-    if (inArr) {
-      if (P.buoy || P.cor || P.damp) rbsc = Q.rhoBS[c];
-      if (P.cor || P.damp) zc = Q.zPos[c];
-      if (P.damp) ztop = Q.zPos[c - k + (P.kMax - 1)];
-    }
-    if (more) issue_aux(i, aux + ((i - i0) & 1) * T::NAUX * T::NT);
-    if (more) issue_ring(i + 1, ns);
-    float rD = 0.0f, rR = 1.0f, rM = 0.0f, rW = 0.0f, rJ = 0.0f;
-    if (more && rtKind) {
-      const long long cr = (long long)(i + 1) * si + rtOff;
-      rD = Q.D[cr]; rR = cur[cr]; rW = cur[3 * n + cr];
-      if (rtKind == 1) { rM = cur[2 * n + cr]; rJ = Q.J32[cr]; }
-      else rJ = Q.J33[cr];
-    }
-
-    // face velocities of this cell (cuda_advectionDevice.cu:89-106)
-    const float dr1 = __fdiv_rn(Dn, w[0][1]);  // D/rho of plane i+1, shared by its three velocities
-    const float cxp1 = contra_dr(dr1, w[1][1], w[3][1], J1n);
-    const float up = (0.5f * dXi) * (cxp1 + cx0);
-    const float* cyP = cs + MSLOTS * PLANE;
-    const float* czP = cyP + T::CYN;
-    const float vm = (0.5f * dYi) * (cyOwn + cyP[ty * MK + tx]);
-    const float vp = (0.5f * dYi) * (cyP[(ty + 2) * MK + tx] + cyOwn);
-    const float wm = (k == P.kMin) ? 0.0f : (0.5f * dZi) * (czOwn + czP[ty * T::CZK + tx]);
-    const float wp = (k + 1 >= P.kMax) ? 0.0f : (0.5f * dZi) * (czP[ty * T::CZK + tx + 2] + czOwn);
-
-    const float J1 = J1c, J2 = J2c, J3 = J3c;
-    const float invD = ax[13 * T::NT];
-    const float r0 = w[0][0];
-    // The moist PGF, Coriolis and Rayleigh terms divide by rho and rho_BS through one correctly
-    // rounded reciprocal per block (phi * (1/rho) instead of phi / rho: within an ulp).
-    float F[8];
-    float fw = 0.0f;  // explicit filter of rho w (filterSelector = 1)
-#pragma unroll
-    for (int s = 0; s < 8; s++) F[s] = 0.0f;
-
-    // pressure-gradient force (cuda_pressureDevice.cu:118-194)
-    if (pgf) {
-      const float* pp = cs + SL_P * PLANE + own;
-      const float dpx = pc1 - ps[SL_P * PLANE + own];
-      const float dpy = pp[PK] - pp[-PK];
-      const float dpz = pp[1] - pp[-1];
-      if (nmoist > 0) {
-        const float rr0 = 1.0f / r0;
-        float rmd = 1.0f;
-        rmd = (float)((double)rmd + (double)(w[SL_QV][0] * rr0) * 1e-3);
-        if (nmoist > 1) rmd = (float)((double)rmd + (double)(w[SL_QL][0] * rr0) * 1e-3);
-        const float rdm = 1.0f / rmd;
-        F[1] = (float)((double)F[1] - (double)rdm * 0.5 * (double)dXi * (double)dpx);
-        F[2] = (float)((double)F[2] - (double)rdm * 0.5 * (double)dYi * (double)dpy);
-        F[3] = (float)((double)F[3] - (double)rdm * 0.5 * (double)(dXi * J1 * dpx + dYi * J2 * dpy + dZi * J3 * dpz));
-      } else {
-        F[1] = F[1] - (0.5f * dXi) * dpx;
-        F[2] = F[2] - (0.5f * dYi) * dpy;
-        F[3] = F[3] - 0.5f * (dXi * J1 * dpx + dYi * J2 * dpy + dZi * J3 * dpz);
-      }
-    }
-
-    // advection of every field (cuda_hydroCoreDevice.cu:631-736; WENO3/WENO5 as x, y, z updates)
-    float fxNext = 0.0f;  // x face of field s + 1 when it was evaluated with field s
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-      if (!f_on<FL>(P, s)) continue;
-      const float* pl = cs + s * PLANE + own;
-      const float z0 = w[s][0];
-      const float xm2 = ns[s * PLANE + own], xm1 = ps[s * PLANE + own];
-      const int sel = f_sel<FL>(P, s);
-      const float bf = adv_split(sel) ? 1.0f : 1.0f - slot_b(P, s);
-      // the x faces of an even and the following odd field as a lane pair when both use the same
-      // packed scheme (compile-time flavours only)
-      float fxp;
-      if (x_paired<FL>(s)) {
-        const int s1 = s + 1;
-        const float bf1 = adv_split(sel) ? 1.0f : 1.0f - slot_b(P, s1);
-        const float2 fx = adv_face2<true>(sel, f2(xm2, ns[s1 * PLANE + own]), f2(xm1, ps[s1 * PLANE + own]),
-                                          f2(z0, w[s1][0]), f2(w[s][1], w[s1][1]), f2(w[s][2], w[s1][2]),
-                                          f2(w[s][3], w[s1][3]), f2s(up), f2(bf, bf1));
-        fxp = fx.x;
-        fxNext = fx.y;
-      } else if (s > 0 && x_paired<FL>(s - 1)) {
-        fxp = fxNext;
-      } else {
-        fxp = adv_face<true>(sel, xm2, xm1, z0, w[s][1], w[s][2], w[s][3], up, bf);
-      }
-      const float pxp = __fmul_rn(up, fxp);
-      const float Dx = __fsub_rn(pxp, xcs[s * T::NT + tid]);
-      xcs[s * T::NT + tid] = pxp;
-      // moist flavours: the two y faces, then the two z faces, as lane pairs (upper face, lower
-      // face) on the packed pipe; the other flavours face by face (their register budget has no
-      // room for the pairs)
-      float Dy, Dz;
-      {
-        const float m3 = pl[-3 * PK], m2 = pl[-2 * PK], m1 = pl[-PK], p1 = pl[PK], p2 = pl[2 * PK], p3 = pl[3 * PK];
-        if constexpr (FL == FL_MOIST || FL == FL_MOIST34) {
-          const float2 v2 = f2(vp, vm);
-          const float2 fy = adv_face2<true>(sel, f2(m2, m3), f2(m1, m2), f2(z0, m1), f2(p1, z0), f2(p2, p1), f2(p3, p2),
-                                            v2, f2s(bf));
-          const float2 py = mul2(v2, fy);
-          Dy = __fsub_rn(py.x, py.y);
-        } else {
-          Dy = vp * adv_face<true>(sel, m2, m1, z0, p1, p2, p3, vp, bf) - vm * adv_face<true>(sel, m3, m2, m1, z0, p1, p2, vm, bf);
-        }
-      }
-      {
-        const float m3 = pl[-3], m2 = pl[-2], m1 = pl[-1], p1 = pl[1], p2 = pl[2], p3 = pl[3];
-        if constexpr (FL == FL_MOIST || FL == FL_MOIST34) {
-          const float2 w2 = f2(wp, wm);
-          const float2 fz = adv_face2<true>(sel, f2(m2, m3), f2(m1, m2), f2(z0, m1), f2(p1, z0), f2(p2, p1), f2(p3, p2),
-                                            w2, f2s(bf));
-          const float2 pz = mul2(w2, fz);
-          Dz = __fsub_rn(pz.x, pz.y);
-        } else {
-          Dz = wp * adv_face<true>(sel, m2, m1, z0, p1, p2, p3, wp, bf) - wm * adv_face<true>(sel, m3, m2, m1, z0, p1, p2, wm, bf);
-        }
-        // the explicit filter of rho w reads the same column; it is added after every other term
-        if (s == 3 && P.filt) fw = filter6_tend(m3, m2, m1, z0, p1, p2, p3, P.filtCoef);
-      }
-      if (adv_split(sel)) {
-        // WENO: x, y and z as three separate updates
-        F[s] = F[s] - invD * Dx;
-        F[s] = F[s] - invD * Dy;
-        F[s] = F[s] - invD * Dz;
-      } else {
-        F[s] = F[s] - invD * (Dx + Dy + Dz);
-      }
-      if (s == 3) {
-        // Rayleigh damping and buoyancy act on F_w right after its advection
-        if (P.damp && inArr) {
-          const float z = zc, zt = ztop;
-          if (z >= (zt - P.dampDepth)) {
-            const float rbs = rbsc, rr0 = 1.0f / r0, rrb = 1.0f / rbs;
-            const float wbs = momentum_bs(P, 3, z, rbs);
-            const float pio2 = 1.5707963267948966f;
-            const double sn = (double)sinf((float)((double)pio2 * (1.0 - (double)((zt - z) / P.dampDepth))));
-            F[3] = (float)((double)F[3] - 0.2 * (double)r0 * (sn * sn) * (double)(w[3][0] * rr0 - wbs * rrb));
-          }
-        }
-        if (P.buoy) {
-          const float rbs = rbsc;
-          if (nmoist > 0) {
-            double rm = (double)r0 + (double)w[SL_QV][0] * 1e-3;
-            if (nmoist == 2) rm += (double)w[SL_QL][0] * 1e-3;
-            const float ratio = r0 / (float)rm;
-            F[3] = (float)((double)F[3] - (double)(ratio * P.g) * (rm - (double)rbs));
-          } else {
-            F[3] = F[3] - P.g * (r0 - rbs);
-          }
-        }
-      }
-    }
-
-    // Coriolis (cuda_coriolisDevice.cu:50-58)
-    if (P.cor && inArr) {
-      const float z = zc, rbs = rbsc;
-      const float ubs = momentum_bs(P, 1, z, rbs), vbs = momentum_bs(P, 2, z, rbs), wbs = momentum_bs(P, 3, z, rbs);
-      const float rr0 = 1.0f / r0, rrb = 1.0f / rbs;
-      const float u0 = w[1][0] * rr0, v0 = w[2][0] * rr0, w0 = w[3][0] * rr0;
-      const float ug = P.fLS * ubs * rrb, vg = P.fLS * vbs * rrb, wg = P.fLS * wbs * rrb;
-      F[1] = F[1] + (P.fHorz * (v0 - vg) - P.fVert * (w0 - wg));
-      F[2] = F[2] - (P.fHorz * (u0 - ug));
-      F[3] = F[3] + (P.fVert * (u0 - ug));
-    }
-
-    if (phys && P.turb && active) {
-      F[1] = F[1] - sg[0];
-      F[2] = F[2] - sg[1];
-      F[3] = F[3] - sg[2];
-      F[4] = F[4] - sg[3];
-      if (tke) F[SL_E] = F[SL_E] + sg[4];
-      if (nmoist > 0 && (P.moistSGS > 0 || P.lsf)) {
-        F[SL_QV] = F[SL_QV] - sg[5];
-        if (nmoist > 1 && P.moistSGS > 0) F[SL_QL] = F[SL_QL] - sg[6];
-      }
-    }
-
-    // saturation adjustment (cuda_moistureDevice.cu:80-247)
-    if (mpStep && active) {
-      const float ri = rinv(r0);
-      const float mth = w[4][0];
-      const float thd = mth * ri;
-      const float prd = P.condBasePres == 1 ? powf(Q.thBS[c] * P.c1, P.cp_cv) : powf(mth * P.c1, P.cp_cv);
-      const float Td = thd * powf(prd / P.p0, P.R_cp);
-      float pvs;
-      const float Tc = fmaxf(-80.0f, (Td - 273.16f));
-      if (Td >= 273.15f) {
-        pvs = (6.11239921f + Tc * (0.443987641f + Tc * (0.142986287e-1f + Tc * (0.264847430e-3f + Tc * (0.302950461e-5f +
-              Tc * (0.206739458e-7f + Tc * (0.640689451e-10f + Tc * (-0.952447341e-13f + -0.976195544e-15f * Tc)))))))) * 100.0f;
-      } else {
-        pvs = (6.11147274f + Tc * (0.503160820f + Tc * (0.188439774e-1f + Tc * (0.420895665e-3f + Tc * (0.615021634e-5f +
-              Tc * (0.602588177e-7f + Tc * (0.385852041e-9f + Tc * (0.146898966e-11f + 0.252751365e-14f * Tc)))))))) * 100.0f;
-      }
-      pvs = fminf((0.99f * prd), pvs);
-      float ffor = 0.0f;
-      const float flim = w[SL_QL][0] * 1e-3f;
-      if (P.moistCond == 1) {
-        ffor = w[SL_QV][0] * 1e-3f - (pvs / (P.R_vapor * Td));
-      } else if (P.moistCond == 2) {
-        const float rv = w[SL_QV][0] * 1e-3f, rvs = pvs / (P.R_vapor * Td);
-        ffor = (rv - rvs) / (1.0f + (powf(P.L_v, 2.0f) * rvs * ri / (P.cp_gas * P.R_vapor * powf(Td, 2.0f))));
-      } else {
-        const float rv = w[SL_QV][0] * 1e-3f;
-        float rvs = pvs / (prd - pvs) / P.Rv_Rg;
-        rvs = rvs / ri;
-        ffor = (rv - rvs) / (1.0f + (powf(P.L_v, 2.0f) * rvs * ri / (P.cp_gas * P.R_vapor * powf(Td, 2.0f))));
-      }
-      float fc = fmaxf(ffor, 0.0f) - fmaxf(fminf(flim, -ffor), 0.0f);
-      fc = fc / P.condTscale;
-      F[SL_QV] = F[SL_QV] - fc * 1e3f;
-      F[SL_QL] = F[SL_QL] + fc * 1e3f;
-      const float prd2 = powf(mth * P.c1, P.cp_cv);
-      const float Td2 = thd * powf(prd2 / P.p0, P.R_cp);
-      F[4] = F[4] + ((thd * P.L_v) / (Td2 * P.cp_gas)) * fc;
-    }
-    // large-scale forcing in the last stage (cuda_hydroCoreDevice.cu:401-406)
-    if (lsfNow && active) lsf_tend(P, Q, c, k, Q.zPos[c], r0, F[1], F[2], F[4], F[SL_QV]);
-    // explicit filter of rho w, every stage, after all other terms (cuda_hydroCoreDevice.cu:414-416)
-    if (P.filt) F[3] = __fadd_rn(F[3], fw);
-
-    if (active) {
-      if (MODE == MODE_FRHS) {
-        frhs[c] = F[0];
-        frhs[n + c] = F[1];
-        frhs[2 * n + c] = F[2];
-        frhs[3 * n + c] = F[3];
-        frhs[4 * n + c] = F[4];
-        if (ntke) frhs[5 * n + c] = F[SL_E];
-        if (nmoist > 0) frhs[(5 + ntke) * n + c] = F[SL_QV];
-        if (nmoist > 1) frhs[(6 + ntke) * n + c] = F[SL_QL];
-      } else {
-        if (STAGE == 2 && frhs) {
-          // the last stage's tendencies, kept when asked (the reference's Frhs after a step)
-          frhs[c] = F[0];
-          frhs[n + c] = F[1];
-          frhs[2 * n + c] = F[2];
-          frhs[3 * n + c] = F[3];
-          frhs[4 * n + c] = F[4];
-          if (ntke) frhs[5 * n + c] = F[SL_E];
-          if (nmoist > 0) frhs[(5 + ntke) * n + c] = F[SL_QV];
-          if (nmoist > 1) frhs[(6 + ntke) * n + c] = F[SL_QL];
-        }
-        // WS2002 RK3 commit (cuda_RKschemes.cu:113-157), rounding as in the cell kernel
-        auto rk = [&](float phi0, float Fv) -> float {
-          if (STAGE == 0) return (float)fma((1.0 / 3.0) * (double)P.dt, (double)Fv, (double)phi0);
-          if (STAGE == 1) return (float)fma(0.5 * (double)P.dt, (double)Fv, (double)phi0);
-          return __fmaf_rn(P.dt, Fv, phi0);
-        };
-        auto b0 = [&](int s) -> float { return same ? w[s][0] : cb[s]; };
-        const long long oq = (5 + ntke) * n;
-        const float a0 = b0(0), a1 = b0(1), a2 = b0(2), a3 = b0(3), a4 = b0(4);
-        const float ae = ntke ? b0(SL_E) : 0.0f;
-        const float aq0 = nmoist > 0 ? b0(SL_QV) : 0.0f;
-        const float aq1 = nmoist > 1 ? b0(SL_QL) : 0.0f;
-        const bool atBot = (k == P.kMin), atTop = (k == P.kMax - 1);
-        Level0 l0{};
-        if (atBot) l0 = level0_inputs(Q, c - k);
-        const float n0 = rk(a0, F[0]);
-        const float n1 = rk(a1, F[1]);
-        const float n2 = rk(a2, F[2]);
-        const float n3 = rk(a3, F[3]);
-        const float n4 = rk(a4, F[4]);
-        const float ne = ntke ? fmaxf(rk(ae, F[SL_E]), 1e-10f) : 0.0f;
-        const float nq0 = nmoist > 0 ? fmaxf(rk(aq0, F[SL_QV]), 0.0f) : 0.0f;
-        const float nq1 = nmoist > 1 ? fmaxf(rk(aq1, F[SL_QL]), 0.0f) : 0.0f;
-        float pn;
-        {
-          float rtm = n4;
-          if (nmoist > 0) rtm = (float)((double)n4 * (1.0 + (double)(P.Rv_Rg * nq0 / n0) * 1e-3));
-          pn = powf(rtm * P.c1, P.cp_cv) - pbs;
-        }
-        const float p0 = atBot ? level0_pressure(P, l0, nmoist, nq0) : 0.0f;
-        // The stores: cells within 3 of an x or y edge also write their periodic images (and,
-        // at the first and last level, the images' halo copies); every other cell writes one
-        // value per field and, at the first and last level, the halo copies below and above.
-        const bool xyEdge = (i < P.iMin + 3) || (i >= P.iMax - 3) || (j < P.jMin + 3) || (j >= P.jMax - 3);
-        if (xyEdge) {
-          store_images(P, nxt, i, j, k, n0, 0, false);
-          store_images(P, nxt + n, i, j, k, n1, atBot ? 3 : 0, false);
-          store_images(P, nxt + 2 * n, i, j, k, n2, atBot ? 3 : 0, false);
-          store_images(P, nxt + 3 * n, i, j, k, n3, atBot ? 3 : 0, false);
-          store_images(P, nxt + 4 * n, i, j, k, n4, 0, false);
-          if (ntke) store_images(P, nxt + 5 * n, i, j, k, ne, atBot ? 3 : 0, false);
-          if (nmoist > 0) store_images(P, nxt + oq, i, j, k, nq0, atBot ? 3 : 0, atTop);
-          if (nmoist > 1) store_images(P, nxt + oq + n, i, j, k, nq1, atBot ? 3 : 0, atTop);
-          store_images(P, pnxt, i, j, k, pn, atBot ? 2 : 0, atTop);
-        } else {
-          nxt[c] = n0;
-          nxt[n + c] = n1;
-          nxt[2 * n + c] = n2;
-          nxt[3 * n + c] = n3;
-          nxt[4 * n + c] = n4;
-          if (ntke) nxt[5 * n + c] = ne;
-          if (nmoist > 0) nxt[oq + c] = nq0;
-          if (nmoist > 1) nxt[oq + n + c] = nq1;
-          pnxt[c] = pn;
-          if (atBot) {
-#pragma unroll
-            for (int h = 1; h <= 3; h++) {
-              nxt[n + c - h] = n1;
-              nxt[2 * n + c - h] = n2;
-              nxt[3 * n + c - h] = n3;
-              if (ntke) nxt[5 * n + c - h] = ne;
-              if (nmoist > 0) nxt[oq + c - h] = nq0;
-              if (nmoist > 1) nxt[oq + n + c - h] = nq1;
-              if (h <= 2) pnxt[c - h] = pn;
-            }
-          }
-          if (atTop) {
-#pragma unroll
-            for (int h = 1; h <= 3; h++) {
-              if (nmoist > 0) nxt[oq + c + h] = nq0;
-              if (nmoist > 1) nxt[oq + n + c + h] = nq1;
-              pnxt[c + h] = pn;
-            }
-          }
-        }
-        if (atBot) store_images(P, pnxt, i, j, 0, p0, 0, false);
-      }
-    }
-
-    // plane i+1 into the other buffer: own values, contravariant velocities, ring tasks
-    float cyN = 0.0f, czN = 0.0f;
+    // face velocities (cuda_advectionDevice.cu:89-106)
+    const float2 r1 = ld2(own1);
+    const float2 dr1 = f2(__fdiv_rn(nD.x, r1.x), __fdiv_rn(nD.y, r1.y));  // D/rho of plane i+1, shared by its three velocities
+    const float2 w1 = ld2(own1 + 3 * T::OWNF);
+    const float2 cx1 = prod2(dr1, fma2(w1, nJ1, ld2(own1 + T::OWNF)));
+    const float2 cyN = prod2(dr1, fma2(w1, nJ2, ld2(own1 + 2 * T::OWNF))), czN = prod2(dr1, prod2(w1, nJ3));
     if (more) {
-#pragma unroll
-      for (int s = 0; s < 8; s++)
-        if (f_on<FL>(P, s)) ns[s * PLANE + own] = w[s][1];
-      if (pgf) ns[SL_P * PLANE + own] = pc1;
-      cyN = contra_dr(dr1, w[2][1], w[3][1], ax[11 * T::NT]);
-      czN = contra_z_dr(dr1, w[3][1], ax[12 * T::NT]);
-      float* v = ns + MSLOTS * PLANE;
-      v[(ty + 1) * MK + tx] = cyN;
-      v[T::CYN + ty * T::CZK + tx + 1] = czN;
-      if (rtKind) v[rtS] = rtKind == 1 ? contra(rD, rR, rM, rW, rJ) : contra_z(rD, rR, rW, rJ);
+      float* v = velB(b ^ 1);
+      st2(v + (ty + 1) * MK + 2 * tx, cyN);
+      st2(v + T::CYN + ty * T::CZP + 2 * tx + 2, czN);
     }
-    // shift the x window and the carried values
-#pragma unroll
-    for (int s = 0; s < 8; s++) {
-#pragma unroll
-      for (int d = 0; d < 3; d++) w[s][d] = w[s][d + 1];
+    const float2 up = mul2(f2s(0.5f * dXi), add2(cx1, cx0));
+    float2 nvm, vp, nwm, wp;  // upper faces, and the lower faces' velocities negated
+    {
+      const float* cy = velB(b) + ty * MK + 2 * tx;
+      const float2 cyO = ld2(cy + MK);
+      nvm = mul2(f2s(-0.5f * dYi), add2(cyO, ld2(cy)));
+      vp = mul2(f2s(0.5f * dYi), add2(ld2(cy + 2 * MK), cyO));
+      const float* cz = velB(b) + T::CYN + ty * T::CZP + 2 * tx + 2;
+      const float2 czO = ld2(cz);
+      const float hz = 0.5f * dZi;
+      const float wl = __fmul_rn(hz, __fadd_rn(czO.x, cz[-1])), wc = __fmul_rn(hz, __fadd_rn(czO.y, czO.x)),
+                  wu = __fmul_rn(hz, __fadd_rn(cz[2], czO.y));
+      // no flow through the first level's lower face and the last level's upper face
+      nwm = f2(atBot ? -0.0f : -wl, -wc);
+      wp = f2(k + 1 >= P.kMax ? 0.0f : wc, k + 2 >= P.kMax ? 0.0f : wu);
     }
-    cx0 = cxp1; upPrev = up;
-    Dc = Dn; J1c = J1n; J2c = ax[11 * T::NT]; J3c = ax[12 * T::NT];
-    cyOwn = cyN; czOwn = czN;
-    float* const t = ps;
-    ps = cs; cs = ns; ns = t;
-    cp_async_wait_all();
+    const float2 niDc = f2(-iD.x, -iD.y);
+    float curB = P.bHyb;
+    Hyb56 hx, hyp, hym, hzp, hzm;
+    auto coefs = [&](float bs) {
+      curB = bs;
+      const float bf = 1.0f - bs;
+      hx = hyb56_coef(up, bf);
+      hyp = hyb56_coef(vp, bf);
+      hym = hyb56_coef(f2(-nvm.x, -nvm.y), bf);
+      hzp = hyb56_coef(wp, bf);
+      hzm = hyb56_coef(f2(-nwm.x, -nwm.y), bf);
+    };
+    coefs(curB);
+
+    // ---- the terms of rho u, rho v, rho w besides advection, SGS mixing and filter
+    float2 G1 = f2s(0.0f), G2 = G1, G3 = G1;
+    {
+      const float2 r0 = ld2(own0), u = ld2(own0 + T::OWNF), v = ld2(own0 + 2 * T::OWNF), w = ld2(own0 + 3 * T::OWNF);
+      float2 rr0 = f2s(0.0f), rdm = f2s(1.0f), qv = rr0, ql = rr0;
+      if (nmoist > 0 || P.cor) rr0 = rcp2(r0);
+      if (nmoist > 0) {
+        // dry-air share rho / (rho + rho q): 1 / (1 + q_v + q_l)
+        qv = ld2(own0 + (5 + ntke) * T::OWNF);
+        if (nmoist > 1) ql = ld2(own0 + (6 + ntke) * T::OWNF);
+        float2 m = fma2(mul2(qv, rr0), f2s(kq), f2s(1.0f));
+        if (nmoist > 1) m = fma2(mul2(ql, rr0), f2s(kq), m);
+        rdm = rcp2(m);
+      }
+      // pressure-gradient force (cuda_pressureDevice.cu:118-194)
+      if (pgf) {
+        const float* q = presB + prs;
+        const float2 a = ld2(q - 2), c = ld2(q), e = ld2(q + 2);
+        const float2 dpx = dif2(pp, pm), dpy = dif2(ld2(q + MRK), ld2(q - MRK));
+        const float2 dpz = f2(__fsub_rn(c.y, a.y), __fsub_rn(e.x, c.x));
+        float2 s = mul2(mul2(f2s(dXi), J1), dpx);
+        s = fma2(mul2(f2s(dYi), J2), dpy, s);
+        s = fma2(mul2(f2s(dZi), J3), dpz, s);
+        const float2 hdx = f2s(-0.5f * dXi), hdy = f2s(-0.5f * dYi);
+        G1 = mul2(hdx, dpx);
+        G2 = mul2(hdy, dpy);
+        G3 = mul2(f2s(-0.5f), s);
+        if (nmoist > 0) {
+          // the product of three rounded once (the reference forms it in double): the rounding error
+          // of the first product is carried
+          const float2 e1 = fma2(hdx, dpx, f2(-G1.x, -G1.y)), e2 = fma2(hdy, dpy, f2(-G2.x, -G2.y));
+          G1 = fma2(rdm, G1, mul2(rdm, e1));
+          G2 = fma2(rdm, G2, mul2(rdm, e2));
+          G3 = mul2(rdm, G3);
+        }
+      }
+      // Rayleigh damping and buoyancy of rho w
+      if (P.damp && active) {
+        G3.x = rayleigh(P, G3.x, z.x, zt, r0.x, w.x);
+        G3.y = rayleigh(P, G3.y, z.y, zt, r0.y, w.y);
+      }
+      if (P.buoy) {
+        float2 d = dif2(r0, rbs);
+        float2 g = f2s(-P.g);
+        if (nmoist > 0) {
+          // excess density rho + rho q - rho_BS, small terms first
+          const float2 low = fma2(f2s(kq), ql, mul2(f2s(kqLo), add2(qv, ql)));
+          d = add2(d, fma2(f2s(kq), qv, low));
+          g = mul2(g, rdm);
+        }
+        G3 = fma2(g, d, G3);
+      }
+      // Coriolis (cuda_coriolisDevice.cu:50-58); the geostrophic wind is V + dV/dz max(z - z_V, 0)
+      if (P.cor) {
+        auto geo = [&](float V, float zg, float gr) -> float2 {
+          return f2(__fmul_rn(P.fLS, z.x < zg ? V : __fmaf_rn(gr, __fsub_rn(z.x, zg), V)),
+                    __fmul_rn(P.fLS, z.y < zg ? V : __fmaf_rn(gr, __fsub_rn(z.y, zg), V)));
+        };
+        const float2 du = dif2(mul2(u, rr0), geo(P.U_g, P.z_Ug, P.Ug_grad));
+        G1 = fma2(f2s(P.fHorz), dif2(mul2(v, rr0), geo(P.V_g, P.z_Vg, P.Vg_grad)), G1);
+        G2 = fma2(f2s(-P.fHorz), du, G2);
+        if (P.fVert != 0.0f) {
+          G1 = fma2(f2s(-P.fVert), mul2(w, rr0), G1);
+          G3 = fma2(f2s(P.fVert), du, G3);
+        }
+      }
+    }
+    // saturation adjustment and inline large-scale forcing of this cell, added to their fields below
+    float2 fcd = f2s(0.0f), fth = fcd, lth = fcd, lqv = fcd;
+    if (mpStep && active) {
+      const float2 r0 = ld2(own0), mth = ld2(own0 + 4 * T::OWNF), qv = ld2(own0 + (5 + ntke) * T::OWNF),
+                   ql = ld2(own0 + (6 + ntke) * T::OWNF);
+      const long long c = po + (long long)j * sj + k;
+      fcd.x = sat_adjust(P, Q, c, r0.x, mth.x, qv.x, ql.x, fth.x);
+      if (both) fcd.y = sat_adjust(P, Q, c + 1, r0.y, mth.y, qv.y, ql.y, fth.y);
+    }
+    if (lsfNow && active) {
+      const float2 r0 = ld2(own0);
+      const long long c = po + (long long)j * sj + k;
+      lsf_tend(P, Q, c, k, Q.zPos[c], r0.x, G1.x, G2.x, lth.x, lqv.x);
+      if (both) lsf_tend(P, Q, c + 1, k + 1, Q.zPos[c + 1], r0.y, G1.y, G2.y, lth.y, lqv.y);
+    }
+    // ---- the fields
+    float2 n0 = f2s(0.0f), n4 = n0, nq = n0;  // new rho, rho theta, rho q_v of the cell
+    const float* xs = sm + own;               // own-cell slots of the field pair
+    float2* xcf = xcs;                        // its carried x fluxes
+    const long long pb = po * 4 + colB, nB = n * 4;
+    const char* bq = (const char*)base + pb;  // its commit base, new values and SGS tendencies (field f - 1)
+    char* vq = (char*)nxt + pb;
+    const char* sq = (const char*)Q.sgsF + (pb - nB);
+    // minus the flux divergence over the cell volume of one field, without the other terms; fw: the
+    // explicit filter of rho w
+    auto divergence = [&](const int f, const int sel, const float* pl, const float* x, float2* xc, float2& fw) -> float2 {
+      float2 acc, px;
+      const float2 z0 = ld2(pl);
+      const float2 m2 = ld2(x + sM2), m1 = ld2(x + sM1), q1 = ld2(x + sP1), q2 = ld2(x + sP2), q3 = ld2(x + sP3);
+      const float2 y3 = ld2(pl - 3 * MRK), y2 = ld2(pl - 2 * MRK), y1 = ld2(pl - MRK), u1 = ld2(pl + MRK),
+                   u2 = ld2(pl + 2 * MRK), u3 = ld2(pl + 3 * MRK);
+      const float2 A = ld2(pl - 4), B = ld2(pl - 2), E = ld2(pl + 2), G = ld2(pl + 4);
+      const float2 xold = *xc;
+      if (sel == ADV_HYB56) {
+        const float2 fx = hyb56_face(hx, z0, dif2(q1, z0), dif2(q2, q1), dif2(q3, q2), dif2(z0, m1), dif2(m1, m2));
+        px = mul2(up, fx);
+        acc = fma2(up, fx, f2(-xold.x, -xold.y));
+        {
+          const float2 d0 = dif2(y2, y3), d1 = dif2(y1, y2), d2 = dif2(z0, y1), d3 = dif2(u1, z0), d4 = dif2(u2, u1), d5 = dif2(u3, u2);
+          acc = fma2(vp, hyb56_face(hyp, z0, d3, d4, d5, d2, d1), acc);
+          acc = fma2(nvm, hyb56_face(hym, y1, d2, d3, d4, d1, d0), acc);
+        }
+        {
+          // differences of neighbouring levels k-3..k+4, then their lane pairs
+          const float a0 = __fsub_rn(B.x, A.y), a1 = __fsub_rn(B.y, B.x), a2 = __fsub_rn(z0.x, B.y), a3 = __fsub_rn(z0.y, z0.x),
+                      a4 = __fsub_rn(E.x, z0.y), a5 = __fsub_rn(E.y, E.x), a6 = __fsub_rn(G.x, E.y);
+          const float2 d0 = f2(a0, a1), d1 = f2(a1, a2), d2 = f2(a2, a3), d3 = f2(a3, a4), d4 = f2(a4, a5), d5 = f2(a5, a6);
+          acc = fma2(wp, hyb56_face(hzp, z0, d3, d4, d5, d2, d1), acc);
+          acc = fma2(nwm, hyb56_face(hzm, f2(B.y, z0.x), d2, d3, d4, d1, d0), acc);
+        }
+      } else {
+        // a field that is zero over the warp's whole stencil (cloud water outside clouds) has zero
+        // fluxes in every scheme; its carried flux is then zero too
+        auto bits = [](float2 v) { return __float_as_uint(v.x) | __float_as_uint(v.y); };
+        const unsigned any = bits(z0) | bits(m2) | bits(m1) | bits(q1) | bits(q2) | bits(q3) | bits(y3) | bits(y2) | bits(y1) |
+                             bits(u1) | bits(u2) | bits(u3) | bits(A) | bits(B) | bits(E) | bits(G) | bits(xold);
+        acc = px = f2s(0.0f);
+        if (__any_sync(0xffffffffu, any << 1)) {
+          const float2 bf = f2s(1.0f - slot_b(P, role_of(f)));
+          const float2 vm = f2(-nvm.x, -nvm.y), wm = f2(-nwm.x, -nwm.y);
+          const float2 fx = adv_face2<true>(sel, m2, m1, z0, q1, q2, q3, up, bf);
+          px = mul2(up, fx);
+          acc = fma2(up, fx, f2(-xold.x, -xold.y));
+          acc = fma2(vp, adv_face2<true>(sel, y2, y1, z0, u1, u2, u3, vp, bf), acc);
+          acc = fma2(nvm, adv_face2<true>(sel, y3, y2, y1, z0, u1, u2, vm, bf), acc);
+          const float2 k2 = f2(B.y, z0.x), k4 = f2(z0.y, E.x);
+          acc = fma2(wp, adv_face2<true>(sel, B, k2, z0, k4, E, f2(E.y, G.x), wp, bf), acc);
+          acc = fma2(nwm, adv_face2<true>(sel, f2(A.y, B.x), B, k2, z0, k4, E, wm, bf), acc);
+        }
+      }
+      if (f == 3 && filt)
+        fw = f2(filter6_tend(A.y, B.x, B.y, z0.x, z0.y, E.x, E.y, P.filtCoef),
+                filter6_tend(B.x, B.y, z0.x, z0.y, E.x, E.y, G.x, P.filtCoef));
+      *xc = px;
+      return acc;
+    };
+    // field pair (f, f + 1); `odd`: only the first exists
+    auto pair = [&](const int f, const int selA, const int selB, const bool odd) {
+      const int rA = role_of(f), rB = role_of(f + 1);
+      // (the bases before the stores: they may alias them)
+      float2 aA = f2s(0.0f), aB = aA, sA = aA, sB = aA;
+      if (MODE != MODE_FRHS) {
+        aA = same ? ld2(xs + s0) : *reinterpret_cast<const float2*>(bq);
+        if (!odd) aB = same ? ld2(xs + s0 + T::OWNF) : *reinterpret_cast<const float2*>(bq + nB);
+      }
+      if ((sgsMask >> f) & 1u) {
+        if constexpr (ANY) sA = g2(Q.sgsF + (long long)(rA == SL_E ? 4 : (rA >= SL_QV ? rA - 1 : f - 1)) * n + po);
+        else sA = *reinterpret_cast<const float2*>(sq);
+      }
+      if ((sgsMask >> (f + 1)) & 1u) {
+        if constexpr (ANY) sB = g2(Q.sgsF + (long long)(rB == SL_E ? 4 : (rB >= SL_QV ? rB - 1 : f)) * n + po);
+        else sB = *reinterpret_cast<const float2*>(sq + nB);
+      }
+      wait(stg, par);
+      const float* pl = sm + T::O_RING + stg * T::STAGE + rng;
+      float2 fw = f2s(0.0f);  // explicit filter of rho w (filterSelector = 1; field 3)
+      if (ANY && selA == ADV_HYB56 && slot_b(P, rA) != curB) coefs(slot_b(P, rA));
+      const float2 dA = divergence(f, selA, pl, xs, xcf, fw);
+      // the TKE's and q_v's b may differ from the hydro fields'
+      if ((ANY || f >= 4) && selB == ADV_HYB56 && !odd && slot_b(P, rB) != curB) coefs(slot_b(P, rB));
+      float2 dB = f2s(0.0f);
+      if (!odd) dB = divergence(f + 1, selB, pl + T::RINGF, xs + T::OWNF, xcf + T::NT, fw);
+      // this warp is done with the pair's stage and oldest slots: the last warp refills them
+      __syncwarp();
+      if ((tid & 31) == 0) {
+        unsigned old;
+        asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;" : "=r"(old) : "r"(tma_smem(cnt + stg)) : "memory");
+        if (old == (unsigned)(T::NW - 1)) {
+          cnt[stg] = 0;
+          int fn = f + 2 * MSTG, in = i;
+          if (fn >= nf) { fn -= (nf + 1) & ~1; in++; }
+          if (in < i1) {
+            const bool pn = pgf && f == 0 && more;
+            tma_bar_expect(bar + stg, ringBytes + (more ? ownBytes : 0u) + (pn ? presBytes : 0u));
+            tma_load4(sm + T::O_RING + stg * T::STAGE, &maps->ring, xk - 4, j0 - 3, in, fn, bar + stg);
+            if (more) tma_load4(sm + sM2 + f * T::OWNF, &maps->own, xk, j0, i + 4, f, bar + stg);
+            if (pn) tma_load3(presB, &maps->pres, xk - 4, j0 - 1, i + 1, bar + stg);
+          }
+        }
+      }
+      if (++stg == MSTG) { stg = 0; par ^= 1u; }
+
+      // the other terms
+      float2 FA = f == 2 ? G2 : f2s(0.0f), FB = f == 0 ? G1 : (f == 2 ? G3 : f2s(0.0f));
+      FA = fma2(niDc, dA, FA);
+      FB = fma2(niDc, dB, FB);
+      FA = fma2(f2s(rA == SL_E ? 1.0f : -1.0f), sA, FA);
+      FB = fma2(f2s(rB == SL_E ? 1.0f : -1.0f), sB, FB);
+      if (mpStep) {
+        if (f == 4) FA = add2(FA, fth);
+        if (rA == SL_QV) FA = fma2(fcd, f2s(-1e3f), FA);
+        if (rB == SL_QV) FB = fma2(fcd, f2s(-1e3f), FB);
+        if (rA == SL_QL) FA = fma2(fcd, f2s(1e3f), FA);
+        if (rB == SL_QL) FB = fma2(fcd, f2s(1e3f), FB);
+      }
+      // large-scale forcing in the last stage (cuda_hydroCoreDevice.cu:401-406)
+      if (lsfNow) {
+        if (f == 4) FA = add2(FA, lth);
+        if (rA == SL_QV) FA = add2(FA, lqv);
+        if (rB == SL_QV) FB = add2(FB, lqv);
+      }
+      // explicit filter of rho w, every stage, after all other terms (cuda_hydroCoreDevice.cu:414-416)
+      if (f == 2 && filt) FB = add2(FB, fw);
+
+      if (keepF && active) {
+        // the tendencies: asked for alone, or the last stage's kept beside the commit (the reference's
+        // Frhs after a step)
+        float* q = reinterpret_cast<float*>((char*)(frhs + f * n) + pb);
+        if (both) st2(q, FA);
+        else q[0] = FA.x;
+        if (!odd) {
+          if (both) st2(q + n, FB);
+          else q[n] = FB.x;
+        }
+      }
+      if (MODE != MODE_FRHS) {
+        float2 vA = STAGE == 0 ? fma2(f2s(chi), FA, fma2(f2s(clo), FA, aA)) : fma2(f2s(chi), FA, aA);
+        float2 vB = STAGE == 0 ? fma2(f2s(chi), FB, fma2(f2s(clo), FB, aB)) : fma2(f2s(chi), FB, aB);
+        if (rA >= SL_QV) vA = max2(vA, 0.0f);
+        if (f >= 4) vB = max2(vB, rB == SL_E ? 1e-10f : 0.0f);
+        if (f == 0) n0 = vA;
+        if (f == 4) n4 = vA;
+        if (rA == SL_QV) nq = vA;
+        if (rB == SL_QV) nq = vB;
+        float* q = reinterpret_cast<float*>(vq);
+        if (pairOut) {
+          st2(q, vA);
+          if (!odd) st2(q + n, vB);
+        }
+        if (oneOut) {
+          q[0] = vA.x;
+          if (!odd) q[n] = vB.x;
+        }
+        // vertical halo copies: below the first level all but rho and rho theta, above the last level moisture
+        if (botOut) {
+          if (f & 2) store_below(q, vA.x, 3);
+          if (!odd) store_below(q + n, vB.x, 3);
+        }
+        if ((ANY || f >= 6) && topOut) {
+          if (rA >= SL_QV) store_above(q, vA, topX);
+          if (!odd && rB >= SL_QV) store_above(q + n, vB, topX);
+        }
+      }
+      xs += 2 * T::OWNF;
+      xcf += 2 * T::NT;
+      bq += 2 * nB; vq += 2 * nB; sq += 2 * nB;
+    };
+    if constexpr (ANY) {
+#pragma unroll 1
+      for (int f = 0; f < nf; f += 2) pair(f, slot_sel(P, role_of(f)), f + 1 < nf ? slot_sel(P, role_of(f + 1)) : 0, f + 1 >= nf);
+    } else {
+      // the hydro fields and TKE in the rolled loop (its end opaque to the compiler, which else unrolls
+      // it), the moisture fields after it with their own schemes, when most face coefficients are dead
+      int nh;
+      asm volatile("mov.u32 %0, %1;" : "=r"(nh) : "n"(6));
+#pragma unroll 1
+      for (int f = 0; f < nh; f += 2) pair(f, ADV_HYB56, ADV_HYB56, false);
+      if constexpr (NF == 8) {
+        if (f_sel<FL>(P, SL_QV) == ADV_HYB56 && slot_b(P, SL_QV) != curB) coefs(slot_b(P, SL_QV));
+        pair(6, f_sel<FL>(P, SL_QV), ADV_WENO5, false);
+      }
+    }
+
+    // the metrics two planes ahead and the ring task's inputs one plane ahead
+    const long long pa = po + 2 * (long long)si;
+    const float2 aD = g2(Q.D + pa), aJ1 = g2(Q.J31 + pa), aJ2 = g2(Q.J32 + pa), aJ3 = g2(Q.J33 + pa), aiD = g2(Q.invD + pa);
+    const float2 ap = pgf ? g2(pcur + pa) : f2s(0.0f);
+    if (more) task_load(i + 1);
+    load_base(i + 1);
+
+    // perturbation pressure of the new state (levels 1..kMin-1 and kMax.. copy their neighbour)
+    if (MODE != MODE_FRHS && active) {
+      const float2 pbs = g2(Q.pBS + po);
+      float2 rtm = n4;
+      if (nmoist > 0)
+        rtm = f2(moist_rth(n4.x, __fdiv_rn(__fmul_rn(P.Rv_Rg, nq.x), n0.x)), moist_rth(n4.y, __fdiv_rn(__fmul_rn(P.Rv_Rg, nq.y), n0.y)));
+      const float2 a = mul2(rtm, f2s(P.c1));
+      const float2 pn = f2(__fsub_rn(powf(a.x, P.cp_cv), pbs.x), __fsub_rn(powf(a.y, P.cp_cv), pbs.y));
+      float* q = reinterpret_cast<float*>((char*)pnxt + pb);
+      if (pairOut) st2(q, pn);
+      if (oneOut) q[0] = pn.x;
+      if (botOut) store_below(q, pn.x, 2);
+      if (topOut) store_above(q, pn, topX);
+    }
+
+    // Cells within 3 of an x or y edge: their periodic images, with the vertical halo copies, from the
+    // values just stored (three fields at a time, their loads in flight together). Kept out of the loop
+    // above, whose body it would double.
+    const bool ilo = i < P.iMin + 3, ihi = i >= P.iMax - 3;
+    if (MODE != MODE_FRHS && active && (ilo || ihi || jlo || jhi)) {
+#pragma unroll 1
+      for (int f = 0; f <= nf; f += 3) {
+        float* q[3];
+        float2 v[3];
+#pragma unroll
+        for (int t = 0; t < 3; t++) {
+          q[t] = reinterpret_cast<float*>((char*)(f + t < nf ? nxt + (f + t) * n : pnxt) + pb);
+          v[t] = both ? ld2(q[t]) : f2s(q[t][0]);
+        }
+#pragma unroll 1
+        for (int m = 0; m < 9; m++) {
+          const int dx = m / 3 - 1, dy = m - 3 * (m / 3) - 1;
+          if (m == 4 || (dx < 0 && !ilo) || (dx > 0 && !ihi) || (dy < 0 && !jlo) || (dy > 0 && !jhi)) continue;
+          const long long o = P.nbr[m] - (long long)dx * P.Nx * si - (long long)dy * P.Ny * sj;
+#pragma unroll
+          for (int t = 0; t < 3; t++) {
+            const int role = f + t < nf ? role_of(f + t) : SL_QL + 1;  // p' last
+            if (f + t > nf) continue;
+            if (both) st2(q[t] + o, v[t]);
+            else q[t][o] = v[t].x;
+            if (atBot && role != 0 && role != 4) store_below(q[t] + o, v[t].x, role > SL_QL ? 2 : 3);
+            if (atTop && role >= SL_QV) store_above(q[t] + o, v[t], topX);
+          }
+        }
+      }
+    }
+    if (more) task_store(velB(b ^ 1));
+    cx0 = cx1;
+    J1 = nJ1; J2 = nJ2; J3 = nJ3; iD = niD;
+    nD = aD; nJ1 = aJ1; nJ2 = aJ2; nJ3 = aJ3; niD = aiD;
+    pm = p0; p0 = pp; pp = ap;
+    const int t = sM2;
+    sM2 = sM1; sM1 = s0; s0 = sP1; sP1 = sP2; sP2 = sP3; sP3 = t;
     __syncthreads();
   }
 }
 
 template <int STAGE, int MODE, int TJ, int FL, int MP = -1>
-__global__ void __launch_bounds__(MK * TJ, 512 / (MK * TJ))
-    k_march(Phys P, Ptrs Q, const float* __restrict__ cur, const float* __restrict__ base, float* __restrict__ nxt,
+__global__ void __launch_bounds__(MT * TJ, march_blocks<TJ>())
+    k_march(const __grid_constant__ Phys P, const __grid_constant__ Ptrs Q, const __grid_constant__ MarchMaps maps,
+            const float* __restrict__ cur, const float* __restrict__ base, float* __restrict__ nxt,
             const float* __restrict__ pcur, float* __restrict__ pnxt, float* __restrict__ frhs, int ni) {
-  march_body<STAGE, MODE, TJ, FL, MP>(P, Q, cur, base, nxt, pcur, pnxt, frhs, ni, blockIdx.x, blockIdx.y, blockIdx.z);
+  march_body<STAGE, MODE, TJ, FL, MP>(P, Q, &maps, cur, base, nxt, pcur, pnxt, frhs, ni, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // One member of a batched launch: its domain, the buffers of the stage, its planes per block and
@@ -854,6 +875,7 @@ __global__ void __launch_bounds__(MK * TJ, 512 / (MK * TJ))
 struct MarchMember {
   Phys P;
   Ptrs Q;
+  const MarchMaps* maps;   // in device memory
   const float *cur, *base, *pcur;
   float *nxt, *pnxt;
   int ni, gx, gy, first;
@@ -863,23 +885,32 @@ struct MarchMember {
 // block b reads its member from the block map, copies that member's parameters into shared memory
 // and runs the member's tile.
 template <int STAGE, int TJ, int FL, int MP = -1>
-__global__ void __launch_bounds__(MK * TJ, 512 / (MK * TJ))
+__global__ void __launch_bounds__(MT * TJ, march_blocks<TJ>())
     k_march_list(const MarchMember* __restrict__ mem, const int* __restrict__ bmap) {
-  __shared__ MarchMember sm_m;
-  __shared__ int sm_idx;
-  const int tid = threadIdx.y * MK + threadIdx.x;
-  if (tid == 0) sm_idx = bmap[blockIdx.x];
-  __syncthreads();
+  extern __shared__ __align__(1024) float sm[];
+  static_assert(march_smem_bytes<TJ, FL>() % alignof(MarchMember) == 0, "parameters follow the tile's plan");
+  MarchMember& sm_m = *reinterpret_cast<MarchMember*>(sm + march_smem_bytes<TJ, FL>() / 4);  // after the tile's plan
+  const int tid = threadIdx.y * MT + threadIdx.x;
   {
-    const int* src = reinterpret_cast<const int*>(mem + sm_idx);
+    const int* src = reinterpret_cast<const int*>(mem + bmap[blockIdx.x]);
     int* dst = reinterpret_cast<int*>(&sm_m);
-    for (int q = tid; q < (int)(sizeof(MarchMember) / sizeof(int)); q += MK * TJ) dst[q] = src[q];
+    for (int q = tid; q < (int)(sizeof(MarchMember) / sizeof(int)); q += MT * TJ) dst[q] = src[q];
   }
   __syncthreads();
   const MarchMember& m = sm_m;
+  if (tid == 0) {
+    tma_map_acquire(&m.maps->ring);
+    tma_map_acquire(&m.maps->own);
+    tma_map_acquire(&m.maps->ownAll);
+    tma_map_acquire(&m.maps->pres);
+    tma_map_acquire(&m.maps->base);
+    tma_map_acquire(&m.maps->sgs);
+    tma_map_acquire(&m.maps->grid);
+    tma_map_acquire(&m.maps->bs);
+  }
   const int local = (int)blockIdx.x - m.first;
   const int bx = local % m.gx, by = (local / m.gx) % m.gy, bz = local / (m.gx * m.gy);
-  march_body<STAGE, MODE_COMMIT, TJ, FL, MP>(m.P, m.Q, m.cur, m.base, m.nxt, m.pcur, m.pnxt, nullptr, m.ni, bx, by, bz);
+  march_body<STAGE, MODE_COMMIT, TJ, FL, MP>(m.P, m.Q, m.maps, m.cur, m.base, m.nxt, m.pcur, m.pnxt, nullptr, m.ni, bx, by, bz);
 }
 
 }  // namespace fe

@@ -4,6 +4,7 @@
 // are compiled in three translation units, one per RK stage (fe_march_s0.cu, fe_march_s1.cu,
 // fe_march_s2.cu), so they build in parallel; the engine calls them through these functions.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include "fe_device.cuh"
@@ -32,6 +33,16 @@ inline int march_flavor(const Phys& P) {
   return FL_ANY;
 }
 
+// Tensor maps of one stage launch at one tile height: the input state's ring tiles (two fields, 40
+// levels by TJ + 6 rows), own-cell tiles (32 by TJ) of two fields and of every field, its p' tiles
+// (40 by TJ + 2), and, as own-cell tiles for L2 prefetches, the commit base, the SGS tendencies, the
+// grid's zPos, J31, J32, J33, D and 1/D together, and the base state one field at a time.
+struct MarchMaps {
+  CUtensorMap ring, own, ownAll, pres, base, sgs, grid, bs;
+};
+cudaError_t march_encode_maps(const Phys& P, const Ptrs& Q, int tj, const float* cur, const float* pcur,
+                              const float* base, MarchMaps* out);
+
 // Whether the last committing stage runs as a pair of kernels (the moist flavours at 8 rows: the
 // kernel of the steps without saturation adjustment carries none of its code).
 inline bool march_split_last_stage(const Phys& P, int tj) {
@@ -42,8 +53,8 @@ inline bool march_split_last_stage(const Phys& P, int tj) {
 // Launch the stage kernel of RK stage STAGE in mode MODE (commit or tendency only) with tiles of
 // tj rows (4 or 8) marching ni planes per thread block.
 template <int STAGE, int MODE>
-void march_launch(const Phys& P, const Ptrs& Q, int tj, int ni, cudaStream_t s, const float* cur, const float* base,
-                  float* nxt, const float* pcur, float* pnxt, float* frhs);
+void march_launch(const Phys& P, const Ptrs& Q, const MarchMaps& maps, int tj, int ni, cudaStream_t s,
+                  const float* cur, const float* base, float* nxt, const float* pcur, float* pnxt, float* frhs);
 
 // Dynamic shared-memory limits of every instantiation of the stage; set on the current device
 // before any launch or capture.

@@ -1,0 +1,65 @@
+// fe_tma.cuh -- tensor-map copies (TMA) and the mbarrier they complete on, as the stage kernel uses
+// them: plain tiled loads into this block's shared memory, no cluster forms.
+#pragma once
+#include <cstdint>
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+namespace fe {
+
+__device__ __forceinline__ uint32_t tma_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void tma_bar_init(uint64_t* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tma_smem(bar)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+__device__ __forceinline__ void tma_bar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tma_smem(bar)), "r"(bytes) : "memory");
+}
+// Bounded wait for the completion of phase `phase`: false when about a second passed. The thread is
+// suspended by the barrier (up to the hinted 20 us a time) instead of spending issue slots on polling.
+__device__ __forceinline__ bool tma_bar_wait(uint64_t* bar, uint32_t phase) {
+  const uint32_t a = tma_smem(bar);
+  for (int t = 0; t < 50000; t++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 20000;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(a), "r"(phase)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+// Tile of a 4-D map (levels, rows, planes, fields) / 3-D map (levels, rows, planes) into shared memory.
+__device__ __forceinline__ void tma_load4(float* dst, const CUtensorMap* map, int x, int y, int z, int w, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+          tma_smem(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(tma_smem(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tma_load3(float* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          tma_smem(dst)),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(tma_smem(bar))
+      : "memory");
+}
+// The same tile into L2 only.
+__device__ __forceinline__ void tma_prefetch4(const CUtensorMap* map, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(map), "r"(x), "r"(y), "r"(z),
+               "r"(w)
+               : "memory");
+}
+__device__ __forceinline__ void tma_prefetch3(const CUtensorMap* map, int x, int y, int z) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(y), "r"(z) : "memory");
+}
+// A map in global memory, written by the host before the launch: make it visible to this thread's copies.
+__device__ __forceinline__ void tma_map_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
+}  // namespace fe

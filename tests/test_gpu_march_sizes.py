@@ -1,0 +1,87 @@
+"""The marching stage kernel where its tiles (32 levels x 8 rows, two levels per thread, up to 16
+planes per block) can go wrong: last levels on either lane of a pair, single-pair and single-row
+remainders, domains narrower than the halo exchange's images, and every planes-per-block choice."""
+import numpy as np
+import pytest
+
+from conftest import interior, rel_l2
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(3, 3, 2), (5, 9, 31), (9, 8, 33), (17, 7, 32), (12, 16, 65), (6, 25, 3)]
+CASES = {"dry": ("cbl_dry", {}), "moist": ("cbl_moist_hill", dict(hill_halfwidth=60.0, hill_height=15.0, qv=(24.0, 8.0, 300.0))),
+         # one species and no TKE advection flavour: the run-time selector form with an odd field count
+         "generic": ("cbl_dry", dict(params={"advectionSelector": 2}))}
+
+
+def _setup(fe, case, size):
+    name, kw = CASES[case]
+    host = fe.cases.setup_host(name, *size, **kw)
+    inp, cfg = host.inputs(), host.config()
+    host.cleanup()
+    rng = np.random.default_rng(sum(size))
+    for f, amp in ((1, 0.5), (2, 0.5), (3, 0.2)):
+        inp["hydroFlds"][f] += (amp * rng.standard_normal(inp["hydroFlds"][f].shape)).astype(np.float32)
+    inp["sgstke"] += (0.1 * rng.random(inp["sgstke"].shape)).astype(np.float32)
+    if inp["moist"] is not None:  # cloud water in part of the domain only: both sides of the zero-field branch
+        inp["moist"][1][..., : size[2] // 2 + 3] += (0.2 * rng.random(inp["moist"][1][..., : size[2] // 2 + 3].shape)).astype(np.float32)
+    return cfg, inp
+
+
+def _domain(fe, cfg, inp):
+    d = fe.Domain(cfg)
+    d.set_inputs(inp)
+    return d
+
+
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_tendencies_match_the_cell_kernel(fe, case, size):
+    """Every stage's tendencies against the one-cell-per-thread kernel, to FP32 rounding of the fluxes:
+    a face value carries about an ulp (6e-8) of the field, a tendency sums six of them over dx."""
+    cfg, inp = _setup(fe, case, size)
+    a, b = _domain(fe, cfg, inp), _domain(fe, cfg, inp)
+    b.set_stage_kernel("cell")
+    for stage in (0, 2):
+        fa, fb = a.build_frhs(stage), b.build_frhs(stage)
+        for key, state in (("hydroFrhs", "hydroFlds"), ("sgstkeFrhs", "sgstke"), ("moistFrhs", "moist")):
+            if fb[key] is None:
+                continue
+            for f in range(fb[key].shape[0]):
+                x, y = interior(fa[key][f]), interior(fb[key][f])
+                flux = float(np.abs(interior(inp[state][f])).max()) * 15.0 * (2 / cfg.dX + 1 / cfg.dZ)
+                tol = 1e-4 * float(np.abs(y).max()) + 6e-7 * flux
+                assert np.abs(x - y).max() <= tol, (key, f, stage, float(np.abs(x - y).max()), tol)
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("size", SIZES)
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_planes_per_block_do_not_change_bits(fe, case, size):
+    """The launched default (planes chosen from the size), explicit shapes and both tile heights: the
+    same state and pressure, halos included; and the pressure a commit writes in the interior columns,
+    level 0 and the halo levels included, equals the one formed afresh from the state (in the halo columns
+    a fresh state's pressure uses the given base state of those columns, a commit's is the periodic image)."""
+    cfg, inp = _setup(fe, case, size)
+    ref = _domain(fe, cfg, inp)
+    ref.advance(9)
+    r = ref.get_state()
+    for tj, ni in ((8, 1), (8, 2), (8, 7), (4, 3)):
+        d = _domain(fe, cfg, inp)
+        d.set_stage_kernel("march", tj, ni)
+        d.advance(9)
+        s = d.get_state()
+        for key in ("hydroFlds", "sgstke", "moist", "pres"):
+            if r[key] is not None:
+                np.testing.assert_array_equal(s[key], r[key], err_msg=f"{key} {tj} {ni}")
+        d.close()
+    fresh = _domain(fe, cfg, inp)
+    fresh.set_state(r["hydroFlds"], r["sgstke"], r["moist"])
+    f = fresh.get_state()
+    for key in ("hydroFlds", "sgstke", "moist"):
+        if r[key] is not None:
+            np.testing.assert_array_equal(f[key], r[key], err_msg=key)
+    np.testing.assert_array_equal(f["pres"][3:-3, 3:-3], r["pres"][3:-3, 3:-3])
+    for d in (ref, fresh):
+        d.close()
