@@ -322,6 +322,22 @@ static int march_planes(long long cols, int nx, long long slots) {
   return best;
 }
 
+// Planes per thread block of the fused SGS kernel (tiles of 32 levels x 8 rows, two blocks per SM): a
+// block costs its planes plus about two to start (four primitive planes and a physics plane), and all
+// blocks take alike, so whole waves count. Measured step times against planes per block: 48x40x32
+// 1: 77 us, 2: 81, 8: 115; 96x96x96 6: 313 us, 8: 333, 12: 303, 16: 326; 128x128x64 8: 365 us, 12: 395,
+// 16: 356; 203x133x75 8: 1027 us, 12: 1001, 16: 1051; 256x256x128 8: 2683 us, 16: 2630, 32: 2688.
+static int sgs_planes(long long cols, int nx, long long slots) {
+  int best = 8;
+  double cost = 1e30;
+  for (int ni : {1, 2, 3, 4, 6, 8, 12, 16, 32}) {
+    const long long waves = (cols * ((nx + ni - 1) / ni) + slots - 1) / slots;
+    const double c = (double)waves * (ni + 2);
+    if (c < cost) { cost = c; best = ni; }
+  }
+  return best;
+}
+
 static int march_attrs();
 static cudaError_t sgs_march_attrs();
 
@@ -362,14 +378,7 @@ extern "C" int fe_create(const fe_config* cfg, int device, fe_domain** out) {
     d->mniDefault = d->mni;
     d->marchSlots = 3 * nsm;
     d->mniAuto = march_planes(cols, P.Nx, d->marchSlots);
-    // fused SGS kernel (tiles of 32 levels x 8 rows, two blocks per SM): the most planes per block
-    // of 64, 32, 16, 8 that still leaves 10 waves
-    d->sgsNi = 8;
-    for (int ni = 64; ni >= 8; ni /= 2)
-      if (cols * ((P.Nx + ni - 1) / ni) >= 20LL * nsm) {
-        d->sgsNi = ni;
-        break;
-      }
+    d->sgsNi = sgs_planes(cols, P.Nx, 2LL * nsm);
     d->lsfBlocks = P.lsfSub ? 2 * nsm : 0;
   }
   rc = march_attrs();
