@@ -77,10 +77,15 @@ int grid_for(const fe_mlp* m, long long tiles, int perSm) {
   return (int)std::max(1LL, std::min(tiles, (long long)m->nsm * perSm));
 }
 
-// gradient of the mean squared standardised error over samples [first, first+count) into m->grad
-int launch_grad(fe_mlp* m, long long first, long long count) {
+int clear_grad(fe_mlp* m) {
   LCU(cudaMemsetAsync(m->grad, 0, sizeof(float) * fe::MP_TOTAL, m->stream));
   LCU(cudaMemsetAsync(m->loss, 0, sizeof(double), m->stream));
+  return FE_OK;
+}
+
+// gradient of the mean squared standardised error over samples [first, first+count) added to the
+// cleared m->grad and m->loss
+int launch_grad(fe_mlp* m, long long first, long long count) {
   const long long tiles = (count + fe::MLP_M - 1) / fe::MLP_M;
   fe::k_mlp_train<<<grid_for(m, tiles, 1), 128, fe::MlpTrainSmem::BYTES, m->stream>>>(
       m->params, m->norm, m->X, m->T, m->order, m->n, first, count, m->grad, m->loss, m->err);
@@ -287,7 +292,8 @@ extern "C" int fe_mlp_gradient(fe_mlp* m, long long first, long long count, floa
   // gradients are taken in data-set order (no shuffling) so callers can reproduce them
   int* saved = m->order;
   m->order = nullptr;
-  int rc = launch_grad(m, first, count);
+  int rc = clear_grad(m);
+  if (!rc) rc = launch_grad(m, first, count);
   m->order = saved;
   if (rc) return rc;
   if (grad) LCU(cudaMemcpyAsync(grad, m->grad, sizeof(float) * fe::MP_TOTAL, cudaMemcpyDeviceToHost, m->stream));
@@ -305,6 +311,7 @@ extern "C" int fe_mlp_train(fe_mlp* m, int steps, long long batch, float lr, dou
   double* dl = nullptr;
   if (loss_hist && steps > 0) LCU(cudaMalloc(&dl, sizeof(double) * steps));
   long long pos = 0;
+  if (int rc = clear_grad(m)) { cudaFree(dl); return rc; }
   for (int s = 0; s < steps; s++) {
     const long long cnt = std::min(batch, m->n);
     int rc = launch_grad(m, pos, cnt);
@@ -314,8 +321,7 @@ extern "C" int fe_mlp_train(fe_mlp* m, int steps, long long batch, float lr, dou
     const float c1 = 1.0f - (float)std::pow((double)b1, (double)m->adamStep);
     const float c2 = 1.0f - (float)std::pow((double)b2, (double)m->adamStep);
     fe::k_adam<<<(fe::MP_TOTAL + 255) / 256, 256, 0, m->stream>>>(m->params, m->grad, m->mom1, m->mom2, lr, b1, b2, eps, c1,
-                                                                   c2);
-    if (dl) cudaMemcpyAsync(dl + s, m->loss, sizeof(double), cudaMemcpyDeviceToDevice, m->stream);
+                                                                   c2, m->loss, dl ? dl + s : nullptr);
   }
   LCU(cudaGetLastError());
   if (dl) {

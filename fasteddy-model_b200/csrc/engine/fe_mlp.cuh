@@ -689,17 +689,25 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(const float* __restrict__ 
 }
 
 // Adam on the FP32 master parameters; padded entries (W1 columns >= 11, W4 rows and b4
-// entries >= 9) stay zero.
-__global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       float lr, float b1, float b2, float eps, float c1, float c2) {
+// entries >= 9) stay zero. Leaves the gradient and the loss cleared for the next step's
+// accumulation and keeps the step's loss in hist (may be nullptr), so that a training step is two
+// launches and nothing else on the stream (a step of 8192 samples is launch-bound).
+__global__ void k_adam(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
+                       float lr, float b1, float b2, float eps, float c1, float c2, double* __restrict__ loss,
+                       double* __restrict__ hist) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e == 0) {
+    if (hist) *hist = *loss;
+    *loss = 0.0;
+  }
   if (e >= MP_TOTAL) return;
   bool pad = false;
   if (e < MP_B1) pad = (e % MLP_K0) >= SGS_NIN;
   else if (e >= MP_W4 && e < MP_B4) pad = ((e - MP_W4) / MLP_H) >= SGS_NOUT;
   else if (e >= MP_B4) pad = (e - MP_B4) >= SGS_NOUT;
-  if (pad) { p[e] = 0.0f; return; }
+  if (pad) { p[e] = 0.0f; g[e] = 0.0f; return; }
   const float gi = g[e];
+  g[e] = 0.0f;
   const float mi = b1 * m[e] + (1.0f - b1) * gi;
   const float vi = b2 * v[e] + (1.0f - b2) * gi * gi;
   m[e] = mi;
